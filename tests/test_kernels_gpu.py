@@ -293,6 +293,30 @@ def test_gemm_plain(ta, tw, tc, T, N, K):
     assert torch.equal(c1[0], c[T // 2])
 
 
+@pytest.mark.parametrize("T", [1, 2, 3, 5, 8, 9, 16, 17, 33, 65, 129, 400])
+@pytest.mark.parametrize("N,K", [(1, 4), (15, 36), (17, 128), (65, 260), (129, 132), (300, 1000), (2700, 64)])
+def test_gemm_float32_tiles(T, N, K):
+    """32-bit operands that 16-byte copies can address: every tile size at its edges (tokens, features, a last partial
+    step along K), and the same bits for a token whatever else is in the batch.  Each result is the sum of
+    four chains of at most K FMAs in all: at most (K + 3) half units of 2^-23 of the sum of the terms' magnitudes off."""
+    from reinfer_b200 import ops
+    a, w = rnd(T, K, dtype=torch.float32, seed=1), rnd(N, K, dtype=torch.float32, seed=2)
+    c = torch.full((T, N), math.nan, device=DEV)
+    ops.gemm_ref(a, w, c)
+    ref, mag = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+    bound = (K + 3) * 2.0 ** -24 * mag
+    assert bool(((c.double() - ref).abs() <= bound).all())
+    base = rnd(T, N + 3, dtype=torch.float32, seed=3)
+    c2 = base.clone()
+    ops.gemm_ref(a, w, c2[:, :N], accumulate=True)
+    assert torch.equal(c2[:, :N], base[:, :N] + c) and torch.equal(c2[:, N:], base[:, N:])
+    for t in (0, T // 2, T - 1):
+        for n in (1, 3, 9, 40):
+            part = torch.empty(min(n, T - t), N, device=DEV)
+            ops.gemm_ref(a[t:t + n], w, part)
+            assert torch.equal(part, c[t:t + n])
+
+
 @pytest.mark.parametrize("h,rows", [(64, 1), (96, 5), (1000, 3), (4096, 2), (5120, 4)])
 @pytest.mark.parametrize("out_dtype,w_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16),
                                                (torch.bfloat16, torch.float32)])
