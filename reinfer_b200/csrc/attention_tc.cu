@@ -3,42 +3,41 @@
 // The formulas are the reference's attention (crates/cuda/kernels/dense_kernels.cu:173-231: scores, causal
 // mask, softmax in float, weighted sum of the values), tiled as flash attention.  A CTA owns 256 query rows: two
 // row tiles A and B of 128 rows each (a row = a token x one of the Gc grouped query heads of one kv head; tile B
-// holds the tokens after tile A's), and walks the request's keys in tiles of 64.  Both row tiles use every key
+// holds the tokens after tile A's), and walks the request's keys in tiles of 128.  Both row tiles use every key
 // tile that comes in, so a key tile is fetched once for 256 rows.  For every key tile j and row tile t
-//     S_t = Q_t K^T        tcgen05.mma, 128 x 64 x 128, operands in shared memory, S in tensor memory (two buffers
-//                          per row tile)
+//     S_t = Q_t K^T        tcgen05.mma, 128 x 128 x 128, operands in shared memory, S in tensor memory
 //     P_t = exp2(S_t - m)  128 threads, one row each (tcgen05.ld gives a thread its whole row: the row maximum and
-//                          sum need no shuffles), P rounded to bfloat16 into shared memory (two buffers per row tile)
-//     O_t += P_t V         tcgen05.mma, 128 x 128 x 64, accumulated in tensor memory over all key tiles: P and O are
+//                          sum need no shuffles), 64 keys at a time, P rounded to bfloat16 into shared memory (a buffer
+//                          per half of the keys and row tile)
+//     O_t += P_t V         tcgen05.mma, 128 x 128 x 64 per half, accumulated in tensor memory over all key tiles: P and O are
 //                          scaled to a maximum that follows the true one only when it rose by more than 2^8 (then the
 //                          row's thread rescales its lane of O in tensor memory, which is rare), so the rows read O once
-// Warp 0 feeds key/value tiles by TMA: ONE request brings the keys (or the values) of a page for this kv head, laid
-// out as [8-key group][64-dim half][8 keys][64 dims] whatever the page size is (the 5-D map of runtime.cu).  Warp 1
+// Warp 0 feeds key/value tiles by TMA, 64 keys at a time: ONE request brings the keys (or the values) of a page for this kv
+// head, laid out as [8-key group][64-dim half][8 keys][64 dims] whatever the page size is (the 5-D map of runtime.cu).  Warp 1
 // allocates tensor memory and issues the scores of tile A, warp 3 those of tile B, warp 2 the weighted sums; warps 4-7 are the rows of tile A,
 // warps 8-11 the rows of tile B.  Q [rows][d], K [keys][d] and P [rows][keys] are K-major operands; V [keys][d] is
 // used as it lands, as an MN-major operand (instruction descriptor bit 16; in the shared-memory descriptor the
 // leading offset steps to the second 64 dims, the stride offset to the next 8 keys) - nothing is transposed.
 //
 // What runs ahead of what.  A hand-over through an mbarrier that a tcgen05.commit arrives at costs well over a
-// thousand clocks from one side's last instruction to the other side's first (measured: the bare skeleton of such
-// hand-overs, with no copy, product or arithmetic in it, ran at 1,700 clocks a key tile).  So no such hand-over may
-// lie on the rows' path from one key tile to the next.  The scores of tile j+2 are issued as soon as the rows have
-// taken the scores of tile j out of tensor memory (they say so at once, before they exponentiate) - not when P(j) is
-// done - by an issuer of their own, so the rows find the next scores waiting; the weighted sums have their own issuer
-// and nothing but the row's last read of O and the reuse of a P buffer two tiles later waits for them.  (Keeping P in
-// tensor memory over the scores it came from - the A operand of the product may lie there - was built and measured:
-// it ties the scores' buffer to the product's completion and was no faster.)
-// What bounds a key tile now (the kernel's own trace, -DRB_TIMELINE: lane 0 of every warp adds up its waits and its
-// work): of the 2,100 cycles a key tile takes, a row warp works 1,970 (the issuers wait for it): 1,270 in P (64
-// scale-and-subtract, exponential, sum, 32 conversions, 8 stores a row), of which 760 are the exponentials' (two row
-// warps share a scheduler's special-function unit).  With the exponentials taken out the tile still takes 1,900: then
-// the rows wait for the scores, whose issuer needs 900 cycles for a tile's 8 products and 2 commits.  Both sides are
-// that close, so neither alone buys much.  Built, measured, left out: two threads per row (half the chain each, the
-// row's maximum agreed through shared memory: 690 against 623 us at 8,192 tokens); a part of the exponentials as a
-// cubic on the FMA pipe (3 of 8: 671 us, 1 of 2: 724 - nine instructions for one); P rounded by integer instructions
-// instead of the conversion (no change).
-// Registers follow the roles (setmaxnreg): 88 for the control warps, 208 for the rows - what the control warps give up
-// (128 threads x 80) must cover what the rows take (256 threads x 40), for the registers come from the CTA's own
+// thousand clocks from one side's last instruction to the other side's first.  So no such hand-over may lie on the rows' path
+// from one key tile to the next.  The rows take all 128 scores into registers at once and say so before they exponentiate:
+// the scores of tile j+1 are issued then and stand ready when the rows come back; the weighted sums have their own issuer
+// and nothing but the row's last read of O and the reuse of a P buffer a tile later waits for them.  Shared memory has no
+// room for a third tile of keys, so what waits for what decides: keys have slots of their own, refilled as soon as the scores
+// that read them are there, a tile ahead of their use; values are refilled behind their product and needed half a tile later.
+//
+// What bounds a key tile now: the special-function units.  A tile's 2 x 128 x 128 exponentials take them 2,048 cycles of the
+// about 3,900 that a tile takes; its products take the tensor cores 2,048.  (-DRB_TIMELINE: lane 0 of every warp adds up its
+// waits and its work; a row warp spends 2,530 in the exponentials' passes, 220 waiting for scores, 230 for its P buffer.)
+// 2,048 tokens behind 14,336 others, 32 query over 8 kv heads: 525 us (980 TFLOP/s); tiles of 64 keys with two score buffers
+// took 663 (a product of 128 x 64 costs nearly what one of 128 x 128 does), 128 keys in one ring of keys and values 642.
+// Scaling, sums and maxima are packed or three-input instructions, and the code of the options is in instantiations of its
+// own, for the rows' loop has to fit the instruction cache: with all options in it, a fifth of the rows' stalls were
+// instruction fetches.  Built, measured, left out: two threads per row (the row's maximum agreed through shared memory: 11 %
+// slower); a part of the exponentials as a cubic on the FMA pipe (8 to 16 % slower); P rounded by integer instructions.
+// Registers follow the roles (setmaxnreg): 64 for the control warps, 216 for the rows - what the control warps give up
+// (128 threads x 104) must cover what the rows take (256 threads x 48), for the registers come from the CTA's own
 // allocation (384 x 168) and a request for more than it holds waits for ever.
 //
 // Options on top: a distance penalty, a learned bias by distance, chunks, a soft cap on the scores (before penalty and
@@ -49,19 +48,21 @@
 #include "sm100.cuh"
 #include <stdlib.h>
 
-#define FC_BN 64                              // keys per tile
+#define FC_BN 64                              // keys per half tile: what one weighted sum takes
+#define FC_KEYS (2 * FC_BN)                   // keys per tile: what one product of scores takes
 #define FC_ROWS 128                           // query rows per row tile
 #define FC_TILES 2                            // row tiles per CTA
 #define FC_D 128
 #define FC_THREADS 384                        // a control group (TMA warp, MMA warp, two idle) and two groups of four row warps
-#define FC_NST 3
-#define FC_KV_BYTES (FC_BN * 256)             // a key (or value) tile: 64 keys x 256 bytes, as 8 groups of [2 halves][8 keys][128 bytes]
+#define FC_SLOTS 6                            // half tiles: keys of even tiles in slots 0, 1, of odd tiles in 2, 3; values in 4, 5
+#define FC_KSLOT(tile) (((tile) & 1) * 2)
+#define FC_VSLOT(half) (4 + ((half) & 1))
+#define FC_KV_BYTES (FC_BN * 256)             // a slot: 64 keys (or values) x 256 bytes, as 8 groups of [2 halves][8 keys][128 bytes]
 #define FC_GROUP 2048                         // bytes from one 8-key group to the next
 #define FC_HALF 1024                          // bytes from a group's first 64 dims to its second
-#define FC_STAGE (2 * FC_KV_BYTES)            // keys and values
 #define FC_QHALF (FC_ROWS * 128)              // 128 rows x 128 bytes: one 64-column half of a Q tile, or one P buffer
 #define FC_RESCALE 8.0f                       // O is brought to a new maximum only when it rose by more than this (log2)
-#define FC_TMEM_COLS 512                      // S: columns 0..255 (tile A buffers 0, 1; tile B buffers 0, 1); O_A 256..383; O_B 384..511
+#define FC_TMEM_COLS 512                      // S_A: columns 0..127; S_B 128..255; O_A 256..383; O_B 384..511
 
 struct FcArgs {
     const bf16* q;
@@ -96,9 +97,10 @@ struct FcArgs {
 };
 
 struct FcShared {
-    unsigned long long full[FC_NST];
-    unsigned long long empty[FC_NST];
-    unsigned long long s_full[FC_TILES][2], s_free[FC_TILES][2], p_full[FC_TILES][2], o_full[FC_TILES][2];
+    unsigned long long full[FC_SLOTS];
+    unsigned long long empty[FC_SLOTS];
+    unsigned long long s_full[FC_TILES], s_free[FC_TILES], p_full[FC_TILES][2], o_full[FC_TILES][2];
+    int uses[FC_SLOTS];                                            // copies issued into each slot
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -148,6 +150,31 @@ __device__ __forceinline__ float fc_ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+// Two floats in a 64-bit register pair, for the packed instructions (one issue slot for two results, each rounded as the
+// scalar instruction rounds it).
+__device__ __forceinline__ unsigned long long fc_pair(float lo, float hi) {
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ void fc_unpair(unsigned long long v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long fc_fma2(unsigned long long x, unsigned long long y, unsigned long long z) {
+    unsigned long long v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(x), "l"(y), "l"(z));
+    return v;
+}
+__device__ __forceinline__ unsigned long long fc_add2(unsigned long long x, unsigned long long y) {
+    unsigned long long v;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(x), "l"(y));
+    return v;
+}
+__device__ __forceinline__ float fc_max3(float x, float y, float z) {
+    float v;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(v) : "f"(x), "f"(y), "f"(z));
+    return v;
 }
 __device__ __forceinline__ uint32_t fc_pack(float lo, float hi) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -200,14 +227,21 @@ extern "C" int rb_fa_tc_trace(unsigned long long* buf) { return (int)cudaMemcpyT
 #define FC_FLUSH(n) do { } while (0)
 #endif
 
+// OPTIONS: which options on the scores there may be (FC_CAP | FC_PENALTY | FC_BIAS).  They are instantiations because their
+// unrolled code would stand in the rows' loop: with all of it there the loop did not fit the instruction cache and the rows
+// spent two fifths of a key tile fetching code that they jumped over.
+#define FC_CAP 1
+#define FC_PENALTY 2
+#define FC_BIAS 4
+template <int OPTIONS>
 __global__ void __launch_bounds__(FC_THREADS, 1)
 fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a) {
     RB_TL(11);
     if (*(volatile int*)&g_rb_kernel_error) return;                // an earlier wait gave up: fail fast, the host sees the word
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    unsigned char* stages = smem;                                  // [FC_NST][keys, values]
-    unsigned char* sQ = stages + FC_NST * FC_STAGE;                // [row tile][two halves of [128 rows][64 dims]]
+    unsigned char* stages = smem;                                  // [FC_SLOTS]
+    unsigned char* sQ = stages + FC_SLOTS * FC_KV_BYTES;           // [row tile][two halves of [128 rows][64 dims]]
     unsigned char* sP = sQ + FC_TILES * 2 * FC_QHALF;              // [row tile][buffer][128 rows][64 keys]
     FcShared* sh = (FcShared*)(sP + FC_TILES * 2 * FC_QHALF);
     const uint32_t stages_u = smem_u32(stages), sQ_u = smem_u32(sQ), sP_u = smem_u32(sP);
@@ -215,17 +249,19 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
     volatile int* abort_flag = &sh->abort_flag;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < FC_NST; ++s) {
+        for (int s = 0; s < FC_SLOTS; ++s) {
             mbar_init(smem_u32(&sh->full[s]), 1);
-            mbar_init(smem_u32(&sh->empty[s]), 3);                 // the issuers' commits: scores of either row tile done (keys), P V done (values)
+            mbar_init(smem_u32(&sh->empty[s]), 2);                 // the issuers' commits: scores (keys) or weighted sums (values) of either row tile done
+            sh->uses[s] = 0;
         }
-        for (int t = 0; t < FC_TILES; ++t)
+        for (int t = 0; t < FC_TILES; ++t) {
+            mbar_init(smem_u32(&sh->s_full[t]), 1);
+            mbar_init(smem_u32(&sh->s_free[t]), 4);                // one arrival per row warp: the scores are in registers
             for (int b = 0; b < 2; ++b) {
-                mbar_init(smem_u32(&sh->s_full[t][b]), 1);
-                mbar_init(smem_u32(&sh->s_free[t][b]), 4);         // one arrival per row warp: the scores are in registers
                 mbar_init(smem_u32(&sh->p_full[t][b]), 4);         // one arrival per row warp: P is written
                 mbar_init(smem_u32(&sh->o_full[t][b]), 1);
             }
+        }
         sh->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -254,7 +290,7 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
         tile -= nt;
     }
     const bool none = e >= a.first_entry + a.n_entries;            // uniform: a CTA beyond the last entry
-    int n_tiles = 0, q0 = 0, n_tok = 0, kv_end = 0, start_pos = 0, tok_base = 0, t_begin = 0, head0 = 0, kh = 0;
+    int n_halves = 0, q0 = 0, n_tok = 0, kv_end = 0, start_pos = 0, tok_base = 0, t_begin = 0, head0 = 0, kh = 0;
     const int* bt = a.block_table;
     if (!none) {
         q0 = tile * tpc;
@@ -269,7 +305,7 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
         int lo_min = a.window > 0 ? max(0, pos_min - a.window + 1) : 0;
         if (a.chunk > 0) lo_min = max(lo_min, pos_min / a.chunk * a.chunk);
         t_begin = lo_min / FC_BN;
-        n_tiles = pos_max / FC_BN + 1 - t_begin;
+        n_halves = pos_max / FC_BN + 1 - t_begin;
         // Q rows (row r of the CTA = token r / Gc, grouped head r % Gc; rows 128.. are tile B) into the swizzled K-major layout
         for (int i = threadIdx.x; i < n_tok * a.Gc * (FC_D / 8); i += FC_THREADS) {
             const int row = i / (FC_D / 8), c = i % (FC_D / 8);
@@ -279,95 +315,99 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
         if (a.window > 0) {
             // With a window the first key tile of a row block may hold pages that went back to the pool: their copies
             // are skipped and their keys masked, but the values at those places are multiplied all the same (by P = 0,
-            // and 0 x NaN is NaN).  So the stages' value halves start as zeros; what a later use leaves there is this
-            // request's own finite data.
-            for (int i = threadIdx.x; i < FC_NST * (FC_KV_BYTES / 16); i += FC_THREADS)
-                *reinterpret_cast<uint4*>(stages + (i / (FC_KV_BYTES / 16)) * FC_STAGE + FC_KV_BYTES + (i % (FC_KV_BYTES / 16)) * 16) = make_uint4(0, 0, 0, 0);
+            // and 0 x NaN is NaN).  So the slots start as zeros; what a later use leaves there is this request's own
+            // finite data.
+            for (int i = threadIdx.x; i < FC_SLOTS * (FC_KV_BYTES / 16); i += FC_THREADS)
+                *reinterpret_cast<uint4*>(stages + i * 16) = make_uint4(0, 0, 0, 0);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
 
-    int issued = 0;                                                // producer: tiles whose copies were issued
+    const int n_tiles = (n_halves + 1) / 2;
     [[maybe_unused]] long long fc_acc[7] = {0, 0, 0, 0, 0, 0, 0};
     if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");           // the control group gives registers up ...
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");           // the control group gives registers up ...
     if (warp == 0) {
-        // ---- producer: runs ahead by up to FC_NST tiles; block-table entries 32 at a time -------------------
+        // ---- producer: the keys of tile i + 1 go out before the values of tile i.  A tile's keys find their slots free as soon as
+        // the scores of two tiles before are there, a tile ahead of their use; values wait for the product of the tile
+        // before, and are needed half a tile after its rows began.  (One ring of six slots in the order of use had the
+        // keys wait for that product too: the rows then waited 800 of 4,700 cycles for their scores.)
+        // Block-table entries 32 at a time.
         const int box_keys = min(a.page_size, FC_BN);              // keys that one request brings
         const int subs = FC_BN / box_keys;
+        const uint32_t lead = lane == 0 ? 1u : 0u;                 // every lane waits, lane 0's requests take effect
         int cached_first = 0, cached = -1;
-        bool have = false;
-        for (int it = 0; it < n_tiles; ++it) {
-            const int s = it % FC_NST;
-            const int k0 = (t_begin + it) * FC_BN;
-            const int pi0 = k0 >> a.page_shift;
-            const int need_last = (k0 + (subs - 1) * box_keys) >> a.page_shift;
-            if (!have || need_last >= cached_first + 32) {
-                cached_first = pi0;
-                cached = (pi0 + lane < a.max_pages) ? bt[pi0 + lane] : -1;
-                have = true;
-            }
-            int pages[8];
-            int n_valid = 0;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int key = k0 + u * box_keys;
-                const int pg = __shfl_sync(0xffffffffu, cached, ((key >> a.page_shift) - cached_first) & 31);
-                pages[u] = (u < subs && key < kv_end) ? pg : -1;
-                n_valid += pages[u] >= 0;
-            }
-            // every lane waits, lane 0's requests take effect (a lane alone inside a branch pays for each of them)
-            const uint32_t lead = lane == 0 ? 1u : 0u;
-            { FC_T0(); if (it >= FC_NST && !fc_wait(smem_u32(&sh->empty[s]), ((it / FC_NST) & 1) ^ 1, abort_flag, 11)) break; FC_ADD(0); }
-            FC_T0();
-            const uint32_t full = smem_u32(&sh->full[s]);
-            mbar_expect_tx_lead(full, (uint32_t)(n_valid * 2 * box_keys * 256), lead);
-            const uint32_t dst0 = stages_u + s * FC_STAGE;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                if (pages[u] >= 0) {
+        bool have = false, ok = true;
+        for (int step = 0; step < 2 * n_tiles + 1 && ok; ++step) { // keys 0; keys 1, values 0; keys 2, values 1; ...
+            const int values = step > 0 && !(step & 1), tile = values ? step / 2 - 1 : (step + 1) / 2;
+            if (tile >= n_tiles) continue;
+#pragma unroll 1
+            for (int half = 2 * tile; half < min(2 * tile + 2, n_halves); ++half) {
+                const int k0 = (t_begin + half) * FC_BN;
+                const int pi0 = k0 >> a.page_shift;
+                const int need_last = (k0 + (subs - 1) * box_keys) >> a.page_shift;
+                if (!have || need_last >= cached_first + 32 || pi0 < cached_first) {
+                    // (values lie up to 192 keys behind the keys that went out before them: 24 pages at most, and a half has 8)
+                    cached_first = max(pi0 - ((3 * FC_BN + a.page_size - 1) >> a.page_shift), 0);
+                    cached = (cached_first + lane < a.max_pages) ? bt[cached_first + lane] : -1;
+                    have = true;
+                }
+                const int s = values ? FC_VSLOT(half) : FC_KSLOT(tile) + (half & 1), use = values ? tile : tile >> 1;
+                { FC_T0(); if (use && !fc_wait(smem_u32(&sh->empty[s]), (uint32_t)((use & 1) ^ 1), abort_flag, 11)) { ok = false; break; } FC_ADD(0); }
+                FC_T0();
+                const uint32_t full = smem_u32(&sh->full[s]);
+                const uint32_t dst0 = stages_u + s * FC_KV_BYTES;
+                // pages of this half that hold keys: a lane each, then one request a page
+                const int my_key = k0 + lane * box_keys;
+                const int my_page = __shfl_sync(0xffffffffu, cached, ((my_key >> a.page_shift) - cached_first) & 31);
+                const uint32_t there = __ballot_sync(0xffffffffu, lane < subs && my_key < kv_end && my_page >= 0);
+                mbar_expect_tx_lead(full, (uint32_t)(__popc(there) * box_keys * 256), lead);
+#pragma unroll 1
+                for (int u = 0; u < subs; ++u) {
+                    const int page = __shfl_sync(0xffffffffu, my_page, u);
+                    if (!((there >> u) & 1u)) continue;
                     const int key = k0 + u * box_keys;
                     const int grp = (key & (a.page_size - 1)) >> 3;          // first 8-key group inside the page
-                    const int j = pages[u] * 2 * a.KH + kh;                 // (page, keys, head); values: + KH
-                    const uint32_t dst = dst0 + (uint32_t)(u * (box_keys >> 3) * FC_GROUP);
-                    tma_load_5d_lead(dst, &map_kv, 0, 0, 0, grp, j, full, lead);
-                    tma_load_5d_lead(dst + FC_KV_BYTES, &map_kv, 0, 0, 0, grp, j + a.KH, full, lead);
+                    tma_load_5d_lead(dst0 + (uint32_t)(u * (box_keys >> 3) * FC_GROUP), &map_kv, 0, 0, 0, grp, (page * 2 + values) * a.KH + kh, full, lead);
                 }
+                if (lead) sh->uses[s] = use + 1;
+                FC_ADD(1);
             }
-            issued = it + 1;
-            FC_ADD(1);
         }
         FC_FLUSH(n_tiles);
     } else if (warp == 1 || warp == 3) {
         // ---- issuers of the scores, one warp per row tile: every lane runs the loop, lane 0's instructions take effect
-        // S_t(i) = Q_t K(i)^T into score buffer i & 1 of row tile t, as soon as the keys have landed and the rows
-        // have taken the scores of two tiles ago out of that buffer: the scores run ahead of the rows, whatever the
-        // products P V are doing.  d = 128 is two 64-column halves of four 16-wide steps each; the keys' 8-row groups
-        // lie 2,048 bytes apart, their second half 1,024 bytes on.  (One warp for both tiles had 16 products and 3
-        // commits to issue per key tile, about 65 cycles each: more than the products take to run.)
+        // S_t(i) = Q_t K(i)^T over the 128 keys of a tile, as soon as the keys have landed and the rows have taken the
+        // scores of the tile before out of tensor memory: the scores run ahead of the rows, whatever the products P V
+        // are doing.  d = 128 is two 64-column halves of four 16-wide steps each; the keys' 8-row groups lie 2,048 bytes
+        // apart (through both slots), their second half 1,024 bytes on.  (One warp for both row tiles had twice the
+        // products and commits to issue, about 65 cycles each: more than the products take to run.)
         const uint32_t lead = lane == 0 ? 1u : 0u;
         const int t = warp == 1 ? 0 : 1;
-        constexpr uint32_t idesc_s = make_idesc(FC_BN);
+        constexpr uint32_t idesc_s = make_idesc(FC_KEYS);
         const uint64_t dq0 = make_smem_desc(sQ_u + (t * 2) * FC_QHALF), dq1 = make_smem_desc(sQ_u + (t * 2 + 1) * FC_QHALF);
         for (int i = 0; i < n_tiles; ++i) {
-            const int s = i % FC_NST;
-            { FC_T0(); if (!fc_wait(smem_u32(&sh->full[s]), (i / FC_NST) & 1, abort_flag, 12)) break; FC_ADD(0); }
-            { FC_T0(); if (i >= 2 && !fc_wait(smem_u32(&sh->s_free[t][i & 1]), (uint32_t)(((i >> 1) & 1) ^ 1), abort_flag, 20)) break; FC_ADD(1); }
+            const int s = FC_KSLOT(i);
+            const bool both = 2 * i + 1 < n_halves;                // (a missing half's scores are never read)
+            const uint32_t par = (uint32_t)((i >> 1) & 1);
+            { FC_T0(); if (!fc_wait(smem_u32(&sh->full[s]), par, abort_flag, 12)) break;
+              if (both && !fc_wait(smem_u32(&sh->full[s + 1]), par, abort_flag, 12)) break; FC_ADD(0); }
+            { FC_T0(); if (i >= 1 && !fc_wait(smem_u32(&sh->s_free[t]), (uint32_t)((i & 1) ^ 1), abort_flag, 20)) break; FC_ADD(1); }
             FC_T0();
             tc_fence_after();
-            const uint32_t sK = stages_u + s * FC_STAGE;
+            const uint32_t sK = stages_u + s * FC_KV_BYTES;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const uint64_t dq = h ? dq1 : dq0;
                 const uint64_t dk = make_smem_desc_lbo_sbo(sK + h * FC_HALF, 16, FC_GROUP);
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
-                    fc_mma_ss(tmem + (uint32_t)((t * 2 + (i & 1)) * FC_BN), dq + (uint64_t)(k * 2), dk + (uint64_t)(k * 2), idesc_s,
-                              (h | k) != 0, lead);
+                    fc_mma_ss(tmem + (uint32_t)(t * FC_KEYS), dq + (uint64_t)(k * 2), dk + (uint64_t)(k * 2), idesc_s, (h | k) != 0, lead);
             }
-            fc_commit_lead(smem_u32(&sh->s_full[t][i & 1]), lead);
-            fc_commit_lead(smem_u32(&sh->empty[s]), lead);         // the keys of this stage are read once these MMAs are done ...
+            fc_commit_lead(smem_u32(&sh->s_full[t]), lead);
+            fc_commit_lead(smem_u32(&sh->empty[s]), lead);         // the keys are read once these MMAs are done
+            if (both) fc_commit_lead(smem_u32(&sh->empty[s + 1]), lead);
             FC_ADD(2);
         }
         FC_FLUSH(n_tiles);
@@ -376,32 +416,32 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
         const uint32_t lead = lane == 0 ? 1u : 0u;
         constexpr uint32_t idesc_mn = make_idesc(FC_D) | (1u << 16);           // B is MN-major
         bool ok = true;
-        for (int it = 0; it < n_tiles && ok; ++it) {
-            const uint32_t sVs = stages_u + (it % FC_NST) * FC_STAGE + FC_KV_BYTES;
-            // V [keys][d] as it lies in the stage is an MN-major operand: a key's 64 dims (128 bytes) contiguous, keys
+        for (int ht = 0; ht < n_halves && ok; ++ht) {
+            const int s = FC_VSLOT(ht);
+            // V [keys][d] as it lies in its slot is an MN-major operand: a key's 64 dims (128 bytes) contiguous, keys
             // 128 bytes apart, groups of 8 keys 2,048 bytes apart (SBO), the second 64 dims 1,024 bytes on (LBO); an
-            // MMA takes 16 keys = two groups.  (The values landed with the keys, which the scores waited for.)
-            const uint64_t dv = make_smem_desc_lbo_sbo(sVs, FC_HALF, FC_GROUP);
+            // MMA takes 16 keys = two groups.
+            const uint64_t dv = make_smem_desc_lbo_sbo(stages_u + s * FC_KV_BYTES, FC_HALF, FC_GROUP);
+            { FC_T0(); if (!fc_wait(smem_u32(&sh->full[s]), (uint32_t)((ht >> 1) & 1), abort_flag, 21)) break; FC_ADD(1); }
 #pragma unroll
             for (int t = 0; t < FC_TILES; ++t) {
-                { FC_T0(); if (!fc_wait(smem_u32(&sh->p_full[t][it & 1]), (it >> 1) & 1, abort_flag, 13)) { ok = false; break; } FC_ADD(0); }
+                { FC_T0(); if (!fc_wait(smem_u32(&sh->p_full[t][ht & 1]), (ht >> 1) & 1, abort_flag, 13)) { ok = false; break; } FC_ADD(0); }
                 FC_T0();
                 tc_fence_after();
-                const uint64_t dp = make_smem_desc(sP_u + (t * 2 + (it & 1)) * FC_QHALF);
+                const uint64_t dp = make_smem_desc(sP_u + (t * 2 + (ht & 1)) * FC_QHALF);
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
-                    fc_mma_ss(tmem + (uint32_t)(FC_TILES * 2 * FC_BN + t * FC_D), dp + (uint64_t)(k * 2),
-                              dv + (uint64_t)(k * ((2 * FC_GROUP) >> 4)), idesc_mn, (it > 0) || k != 0, lead);
-                fc_commit_lead(smem_u32(&sh->o_full[t][it & 1]), lead);
+                    fc_mma_ss(tmem + (uint32_t)(FC_TILES * FC_KEYS + t * FC_D), dp + (uint64_t)(k * 2),
+                              dv + (uint64_t)(k * ((2 * FC_GROUP) >> 4)), idesc_mn, (ht > 0) || k != 0, lead);
+                fc_commit_lead(smem_u32(&sh->o_full[t][ht & 1]), lead);
+                fc_commit_lead(smem_u32(&sh->empty[s]), lead);     // the values of this slot are read once these are done (for either row tile)
                 FC_ADD(2);
             }
-            if (!ok) break;
-            fc_commit_lead(smem_u32(&sh->empty[it % FC_NST]), lead);   // ... and its values once these are
         }
         FC_FLUSH(n_tiles);
     }
     } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");      // ... and the rows take them
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");      // ... and the rows take them
         // ---- softmax rows: thread = row = tensor-memory lane; group t owns row tile t through all key tiles ----------
         const int t = (warp - 4) >> 2;
         const int quad = warp & 3;                                 // the lanes this warp may read: 32 * (warp % 4) ..
@@ -412,54 +452,45 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
         int lo = a.window > 0 ? max(0, pos - a.window + 1) : 0;
         if (a.chunk > 0) lo = max(lo, max(pos, 0) / a.chunk * a.chunk);
         // the distance penalty of this row's head, in units of the raw score (the scale is applied to the difference)
-        const bool pen = a.r1 != nullptr;
+        const bool pen = (OPTIONS & FC_PENALTY) && a.r1 != nullptr;
         const float pen_a = pen ? a.r1[head0 + row % a.Gc] / a.scale_log2 : 0.0f, pen_b = pen ? a.r2[head0 + row % a.Gc] : 0.0f;
         // the bias by distance of this row's head, in units of the raw score like the penalty; a tile whose keys all lie
         // at least bias_last behind the row gets one constant
-        const float* brow = a.bias ? a.bias + (size_t)(head0 + row % a.Gc) * (a.bias_last + 1) : nullptr;
+        const float* brow = (OPTIONS & FC_BIAS) && a.bias ? a.bias + (size_t)(head0 + row % a.Gc) * (a.bias_last + 1) : nullptr;
         const float bias_unit = 1.4426950408889634f / a.scale_log2;
         const float bias_far = brow ? brow[a.bias_last] * bias_unit : 0.0f;
         // m: the maximum that P and O are scaled to (it follows the true maximum only in steps larger than
         // FC_RESCALE, so that O can stay in tensor memory and be accumulated by the MMA itself); l: the sum in that scale
         float m = -INFINITY, l = 0.0f;
         const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
-        const uint32_t o_col = (uint32_t)(FC_TILES * 2 * FC_BN + t * FC_D);
+        const uint32_t o_col = (uint32_t)(FC_TILES * FC_KEYS + t * FC_D);
         bool ok = true;
-        for (int it = 0; it < n_tiles; ++it) {
-            const int s = it % FC_NST, b = it & 1;
-            const uint32_t par = (uint32_t)((it >> 1) & 1);
-            const int k0 = (t_begin + it) * FC_BN;
-            if (t == 0 && k0 + FC_BN > kv_end) {
-                // the request's last tile: slots of its last page beyond its length hold foreign data - the values
-                // there are zeroed before the tensor core multiplies them (by P = 0, but 0 x NaN is NaN).  The rows of
-                // tile A do it; the product of tile B is issued behind A's, so it sees the zeros too.
-                if (!fc_wait(smem_u32(&sh->full[s]), (it / FC_NST) & 1, abort_flag, 14)) { ok = false; break; }
-                unsigned char* sV = stages + s * FC_STAGE + FC_KV_BYTES;
-                for (int i = row; i < FC_BN * 16; i += FC_ROWS) {
-                    const int r = i / 16, c = i % 16;
-                    if (k0 + r >= kv_end) *reinterpret_cast<uint4*>(sV + fc_kv_off(r, c)) = make_uint4(0, 0, 0, 0);
-                }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the zeros, before the tensor core reads the values
-            }
-            // S: this row's 64 scores in one go (one wait for tensor memory); maxima and sums in four independent chains
-            { FC_T0(); if (!fc_wait(smem_u32(&sh->s_full[t][b]), par, abort_flag, 15)) { ok = false; break; } FC_ADD(0); }
+        for (int it = 0; it < n_tiles && ok; ++it) {
+            // S: this row's 128 scores in one go (one wait for tensor memory); then the next tile's may come
+            uint32_t s_all[FC_KEYS];
+            { FC_T0(); if (!fc_wait(smem_u32(&sh->s_full[t]), (uint32_t)(it & 1), abort_flag, 15)) { ok = false; break; } FC_ADD(0); }
 #ifdef RB_TIMELINE
             const long long fc_tile0 = clock64();
 #endif
             tc_fence_after();
-            const bool edge = k0 + FC_BN - 1 > pos || k0 < lo;     // the tile crosses this row's causal edge or window
-            uint32_t sr[FC_BN];
-            const uint32_t s_col = (uint32_t)((t * 2 + b) * FC_BN);
 #pragma unroll
-            for (int c = 0; c < FC_BN / 16; ++c) tc_ld16(lane_base + s_col + (uint32_t)(c * 16), sr + c * 16);
+            for (int c = 0; c < FC_KEYS / 16; ++c) tc_ld16(lane_base + (uint32_t)(t * FC_KEYS + c * 16), s_all + c * 16);
             tc_ld_wait();
 #ifdef RB_TIMELINE
             fc_acc[1] += clock64() - fc_tile0;
 #endif
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&sh->s_free[t][b]));          // this buffer may take the scores of tile it + 2
-            if (a.cap_raw > 0.0f) {
+            if (lane == 0) mbar_arrive(smem_u32(&sh->s_free[t]));
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {                          // 64 keys at a time: P, and the weighted sum that may begin on it
+            if (2 * it + b >= n_halves) break;
+            uint32_t* sr = s_all + b * FC_BN;
+            const int k0 = (t_begin + 2 * it + b) * FC_BN;
+            const uint32_t par = (uint32_t)(it & 1);
+            const bool edge = k0 + FC_BN - 1 > pos || k0 < lo;     // these keys cross this row's causal edge or window
+            const bool begins = it == 0 && b == 0;
+            if ((OPTIONS & FC_CAP) && a.cap_raw > 0.0f) {
                 // tanh z = 1 - 2 / (e^(2z) + 1): one exponential and one reciprocal of the special-function unit, exact
                 // at both ends (e = inf gives 1, e = 0 gives -1); the error is an absolute 2^-23 or so of the cap
 #pragma unroll
@@ -494,74 +525,98 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
                     if (key < lo || key > pos) sr[j] = 0xff800000u;            // -inf
                 }
             }
-            // this P buffer was read by the product of two key tiles ago, which must be done before it is written again
-            if (it >= 2) {
+            // this P buffer was read by the product of the key tile before, which must be done before it is written again
+            if (it >= 1) {
                 FC_T0();
                 if (!fc_wait(smem_u32(&sh->o_full[t][b]), par ^ 1, abort_flag, 16)) { ok = false; break; }
                 FC_ADD(2);
             }
+            if (t == 0 && k0 + FC_BN > kv_end) {
+                // the request's last keys: slots of its last page beyond its length hold foreign data - the values
+                // there are zeroed before the tensor core multiplies them (by P = 0, but 0 x NaN is NaN).  The rows of
+                // tile A do it; the product of tile B is issued behind A's, so it sees the zeros too.  (Behind the wait above: the
+                // product of the tile before has then read this slot, so its barrier cannot be two phases behind.)
+                const int s = FC_VSLOT(b);
+                if (!fc_wait(smem_u32(&sh->full[s]), par, abort_flag, 14)) { ok = false; break; }
+                unsigned char* sV = stages + s * FC_KV_BYTES;
+                for (int i = row; i < FC_BN * 16; i += FC_ROWS) {
+                    const int r = i / 16, c = i % 16;
+                    if (k0 + r >= kv_end) *reinterpret_cast<uint4*>(sV + fc_kv_off(r, c)) = make_uint4(0, 0, 0, 0);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the zeros, before the tensor core reads the values
+            }
             unsigned char* sPb = sP + (t * 2 + b) * FC_QHALF;
-            // P = 2^(S * scale - base), rounded to bfloat16, into the buffer; and its row sum
+            // P = 2^(S * scale - base), rounded to bfloat16, into the buffer; its row sum; and, beside the exponentials (nothing
+            // here waits for it), the maximum of the raw scores in `top`
+            float top = -INFINITY;
             auto emit = [&](float base) -> float {
-                float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                unsigned long long sum2[2] = {0ull, 0ull};             // four running sums, packed in pairs
+                float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+                const unsigned long long scale2 = fc_pair(a.scale_log2, a.scale_log2), base2 = fc_pair(-base, -base);
 #pragma unroll
                 for (int c = 0; c < FC_BN / 8; ++c) {
                     float p[8];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) { p[j] = fc_ex2(fmaf(__uint_as_float(sr[c * 8 + j]), a.scale_log2, -base)); sum4[j & 3] += p[j]; }
+                    for (int j = 0; j < 8; j += 2) {
+                        const float s0 = __uint_as_float(sr[c * 8 + j]), s1 = __uint_as_float(sr[c * 8 + j + 1]);
+                        mx4[j >> 1] = fc_max3(mx4[j >> 1], s0, s1);
+                        fc_unpair(fc_fma2(fc_pair(s0, s1), scale2, base2), p[j], p[j + 1]);
+                        p[j] = fc_ex2(p[j]);
+                        p[j + 1] = fc_ex2(p[j + 1]);
+                        sum2[(j >> 1) & 1] = fc_add2(sum2[(j >> 1) & 1], fc_pair(p[j], p[j + 1]));
+                    }
                     uint4 pk;
                     pk.x = fc_pack(p[0], p[1]); pk.y = fc_pack(p[2], p[3]); pk.z = fc_pack(p[4], p[5]); pk.w = fc_pack(p[6], p[7]);
                     *reinterpret_cast<uint4*>(sPb + fc_off(row, c, 0)) = pk;
                 }
-                return (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+                top = fmaxf(fc_max3(mx4[0], mx4[1], mx4[2]), mx4[3]);
+                float s0, s1, s2, s3;
+                fc_unpair(sum2[0], s0, s1);
+                fc_unpair(sum2[1], s2, s3);
+                return (s0 + s1) + (s2 + s3);
             };
             // The scale m follows the true maximum only when that rose by more than FC_RESCALE (P then stays below
             // 2^FC_RESCALE, which bfloat16 and the float accumulators hold as well as values below 1).  So in nearly every
             // tile the old scale stays, and the exponentials need not wait for this tile's maximum: both are computed side
             // by side, and only a warp in which some row's scale has to move (always in a row's first tile) does its
             // exponentials again.
-            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#ifdef RB_TIMELINE
-            const long long fc_c3 = clock64();
-#endif
-#pragma unroll
-            for (int j = 0; j < FC_BN; ++j) mx4[j & 3] = fmaxf(mx4[j & 3], __uint_as_float(sr[j]));
-            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * a.scale_log2;   // the scale is positive
-            float sum = 0.0f;
 #ifdef RB_TIMELINE
             const long long fc_c5 = clock64();
-            fc_acc[3] += fc_c5 - fc_c3;
 #endif
-            if (it > 0) sum = emit(m == -INFINITY ? 0.0f : m);
-#ifdef RB_TIMELINE
-            fc_acc[5] += clock64() - fc_c5;
-#endif
-            const bool moves = (m == -INFINITY) ? (mx != -INFINITY) : (mx > m + FC_RESCALE);
-            if (it == 0 || __any_sync(0xffffffffu, moves)) {
+            // (one copy of the exponentials' code, run once or twice: see OPTIONS)
+            float sum = 0.0f;
+#pragma unroll 1
+            for (int again = 0; ; ++again) {
+                sum = emit(m == -INFINITY ? 0.0f : m);
+                const float mx = top * a.scale_log2;               // the scale is positive
+                const bool moves = (m == -INFINITY) ? (mx != -INFINITY) : (mx > m + FC_RESCALE);
+                if (again || !__any_sync(0xffffffffu, moves)) break;
                 float alpha = 1.0f;
                 if (m == -INFINITY) m = mx;
                 else if (moves) { alpha = fc_ex2(m - mx); m = mx; }
-                if (it >= 1 && __any_sync(0xffffffffu, alpha != 1.0f)) {
-                    // rare: O = O * alpha in tensor memory, every lane of the warp with its own factor (1 for most); the
-                    // product of the key tile before (the last one that can have been issued) must have landed in O first
-                    if (!fc_wait(smem_u32(&sh->o_full[t][b ^ 1]), (uint32_t)(((it - 1) >> 1) & 1), abort_flag, 18)) { ok = false; break; }
-                    tc_fence_after();
-#pragma unroll
-                    for (int c = 0; c < FC_D / 32; ++c) {
-                        uint32_t ov[32];
-                        tc_ld16(lane_base + o_col + (uint32_t)(c * 32), ov);
-                        tc_ld16(lane_base + o_col + (uint32_t)(c * 32 + 16), ov + 16);
-                        tc_ld_wait();
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) ov[j] = __float_as_uint(__uint_as_float(ov[j]) * alpha);
-                        fc_st16(lane_base + o_col + (uint32_t)(c * 32), ov);
-                        fc_st16(lane_base + o_col + (uint32_t)(c * 32 + 16), ov + 16);
-                    }
-                    fc_st_wait();
-                }
                 l *= alpha;
-                sum = emit(m == -INFINITY ? 0.0f : m);
+                if (begins || !__any_sync(0xffffffffu, alpha != 1.0f)) continue;
+                // rare: O = O * alpha in tensor memory, every lane of the warp with its own factor (1 for most); the
+                // product of the 64 keys before (the last one that can have been issued) must have landed in O first
+                if (!fc_wait(smem_u32(&sh->o_full[t][b ^ 1]), (uint32_t)((b ? it : it - 1) & 1), abort_flag, 18)) { ok = false; break; }
+                tc_fence_after();
+#pragma unroll 1
+                for (int c = 0; c < FC_D / 32; ++c) {
+                    uint32_t ov[32];
+                    tc_ld16(lane_base + o_col + (uint32_t)(c * 32), ov);
+                    tc_ld16(lane_base + o_col + (uint32_t)(c * 32 + 16), ov + 16);
+                    tc_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) ov[j] = __float_as_uint(__uint_as_float(ov[j]) * alpha);
+                    fc_st16(lane_base + o_col + (uint32_t)(c * 32), ov);
+                    fc_st16(lane_base + o_col + (uint32_t)(c * 32 + 16), ov + 16);
+                }
+                fc_st_wait();
             }
+            if (!ok) break;
+#ifdef RB_TIMELINE
+            fc_acc[5] += clock64() - fc_c5;
+#endif
             l += sum;
 #ifdef RB_TIMELINE
             const long long fc_c6 = clock64();
@@ -572,13 +627,16 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
             if (lane == 0) mbar_arrive(smem_u32(&sh->p_full[t][b]));
 #ifdef RB_TIMELINE
             fc_acc[6] += clock64() - fc_c6;
+#endif
+            }
+#ifdef RB_TIMELINE
             fc_acc[4] += clock64() - fc_tile0;
 #endif
         }
         FC_FLUSH(n_tiles);
         // the row of O, once the tile's last products are done (the last one on each of the two barriers)
         if (ok && n_tiles > 0) {
-            const int last = n_tiles - 1;
+            const int last = n_halves - 1;
             ok = fc_wait(smem_u32(&sh->o_full[t][last & 1]), (uint32_t)((last >> 1) & 1), abort_flag, 17);
             if (ok && last >= 1) ok = fc_wait(smem_u32(&sh->o_full[t][(last - 1) & 1]), (uint32_t)(((last - 1) >> 1) & 1), abort_flag, 19);
         }
@@ -622,8 +680,8 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
     __syncthreads();
     if (*abort_flag && threadIdx.x == 0) {
         // copies that were issued but never consumed still write this CTA's shared memory: wait for them
-        for (int it = max(0, issued - FC_NST); it < issued; ++it)
-            mbar_drain(smem_u32(&sh->full[it % FC_NST]), (it / FC_NST) & 1);
+        for (int s = 0; s < FC_SLOTS; ++s)
+            if (sh->uses[s]) mbar_drain(smem_u32(&sh->full[s]), (uint32_t)((sh->uses[s] - 1) & 1));
     }
     __syncthreads();
     if (warp == 1) {
@@ -666,15 +724,15 @@ extern "C" int rb_fa_prefill_tc(const void* q, const void* cache, long long num_
     a.sink = sink; a.gate = gate; a.gate_stride = gate_stride; a.gate_heads = gate_heads;
     CUtensorMap map;
     if (rb_tensor_map_kv_pages(cache, num_pages, KH, page_size, &map)) return -1;
-    constexpr size_t smem = (size_t)FC_NST * FC_STAGE + FC_TILES * 4 * FC_QHALF + sizeof(FcShared) + 1024;
-    static bool done = false;
-    if (!done) {
-        cudaError_t e = cudaFuncSetAttribute(fa_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        done = true;
-    }
+    constexpr size_t smem = (size_t)FC_SLOTS * FC_KV_BYTES + FC_TILES * 4 * FC_QHALF + sizeof(FcShared) + 1024;
+    static_assert(smem <= 232448, "more than the shared memory of an SM");
     if (n_tiles > 65535) RB_REFUSE("attention (tcgen05): %d row tiles in one launch", n_tiles);
-    return rb_launch(fa_prefill_tc_kernel, dim3(KH * a.chunks, n_tiles), dim3(FC_THREADS), smem, (cudaStream_t)stream, map, a);
+    const int options = (softcap > 0.0f ? FC_CAP : 0) | (r1 ? FC_PENALTY : 0) | (bias ? FC_BIAS : 0);
+    auto kernel = options == 0 ? fa_prefill_tc_kernel<0> : options == FC_CAP ? fa_prefill_tc_kernel<FC_CAP> : options == FC_PENALTY ? fa_prefill_tc_kernel<FC_PENALTY> :
+        options == FC_BIAS ? fa_prefill_tc_kernel<FC_BIAS> : fa_prefill_tc_kernel<FC_CAP | FC_PENALTY | FC_BIAS>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
+    return rb_launch(kernel, dim3(KH * a.chunks, n_tiles), dim3(FC_THREADS), smem, (cudaStream_t)stream, map, a);
 }
 
 // The group of query heads that share a CTA's rows, as rb_fa_prefill_tc chooses it, and the rows of a CTA (for the

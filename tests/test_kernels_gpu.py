@@ -658,6 +658,33 @@ def test_paged_attention_plain(QH, KH, d, page, dtype, window):
     assert (out.double().cpu() - ref).abs().max().item() <= tol * ref.abs().max().item()
 
 
+@pytest.mark.parametrize("QH,KH", [(64, 8), (32, 8), (8, 8), (16, 1)])
+@pytest.mark.parametrize("lens,q_lens", [([1980, 700], [1000, 700]), ([2047], [2047]), ([1153, 129, 64], [130, 129, 64])])
+def test_prompt_attention_ends_anywhere_in_a_tile(QH, KH, lens, q_lens):
+    """The tcgen05 attention where a request's keys end in either half of a 128-key tile, after many tiles and after one, three
+    times over (its warps run far ahead of one another: what reads a slot too early does not do so every time).  P and the
+    results are rounded to bfloat16, here and in the kernel it is held to: three half units of 2^-8 of the largest value."""
+    from reinfer_b200 import ops
+    d, page, g = 128, 16, torch.Generator(device=DEV).manual_seed(5)
+    pages = [-(-n // page) for n in lens]
+    cache = torch.randn(sum(pages) + 1, 2, KH, page, d, generator=g, device=DEV).to(torch.bfloat16)
+    bt = torch.full((len(lens), max(pages)), -1, dtype=torch.int32)
+    for r, n in enumerate(pages):
+        bt[r, :n] = torch.arange(sum(pages[:r]), sum(pages[:r]) + n)
+    bt, q = bt.to(DEV), (1.5 * torch.randn(sum(q_lens), QH, d, generator=g, device=DEV)).to(torch.bfloat16)
+    as_int = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    ref = torch.empty_like(q)
+    ops.paged_attention_ref(q, cache, bt, as_int([r for r, n in enumerate(q_lens) for _ in range(n)]),
+                            as_int([p for l, n in zip(lens, q_lens) for p in range(l - n, l)]), ref, QH, KH, d, page, 0, d ** -0.5)
+    bound = 3 * 2.0 ** -9 * cache.float().abs().max().item()
+    for _ in range(3):
+        out = torch.full_like(q, math.nan)
+        ops.fa_prefill_tc(q, cache, bt, as_int([sum(q_lens[:r]) for r in range(len(lens) + 1)]), as_int(lens), out, 0, len(lens), q_lens,
+                          QH, KH, d, page, 0, d ** -0.5)
+        assert (out.float() - ref.float()).abs().max().item() <= bound
+    assert ops.kernel_error() == 0
+
+
 def test_attention_finds_one_far_key():
     """One key among hundreds gets a score that stands out; the output must be its value."""
     from reinfer_b200 import ops
