@@ -651,7 +651,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     // epilogue writes 16 features of it at a time.  Fewer rows leave room for a stage more.
     constexpr bool DUAL = MODE == 1, FLIP = MODE != 0, HEADS = MODE == 3;
     static_assert(!HEADS || ROWS == 2 * TC_BM, "two heads of 128 a tile");
-    static_assert(ROWS % 32 == 0 && ROWS >= 32 && ROWS <= 2 * TC_BM, "rows of the N operand");
+    static_assert(ROWS % (DUAL ? 32 : 16) == 0 && ROWS >= 32 && ROWS <= 2 * TC_BM, "rows of the N operand");
     constexpr int FEATS = (MODE == 2 || MODE == 3) ? ROWS : MODE == 1 ? ROWS / 2 : TC_BM;   // features per tile
     RB_TL(DUAL ? 9 : 8);
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -1448,11 +1448,18 @@ static int g_tc_gated_stream = 1;
 // 0 = the kernel with a feature per lane (128 + 128 rows a CTA).  Returns the old value.
 extern "C" int rb_set_gemm_gated_stream(int v) { int old = g_tc_gated_stream; g_tc_gated_stream = v ? 1 : 0; return old; }
 
+// Weight rows per tile of the token-lane forms, the stages that fit beside them, and the nanoseconds that a 64-deep k-step
+// takes a CTA then (tiles of T = 2,048 x N = 2,560 and 4,096, K = 9,728 and 12,288, divided by rounds and k-steps).  A step's
+// time falls much slower than its width: issuing its products and its trip through the barriers stay.  So the widest tile is
+// the best as long as the tiles come out even over the SMs, and a narrow one where they do not: 2,560 features over 2,048
+// tokens are 160 tiles of 256 (118 us at K = 9,728), 192 of 224 (103 us), 288 of 144 (95 us) on 148 SMs.
+static const struct { int rows; double ns; } TC_WIDTHS[] = {{256, 400.0}, {224, 335.0}, {192, 325.0}, {160, 314.0}, {144, 300.0}, {64, 268.0}};
 static int g_tc_tile_feats = 0;
-// Weight rows per tile of the token-lane forms: 0 = chosen per product, 256 (four stages) or 224 (five).  Returns the old value.
+// 0 = chosen per product, or one of TC_WIDTHS.  Returns the old value.
 extern "C" int rb_set_gemm_tile_features(int v) {
     int old = g_tc_tile_feats;
-    g_tc_tile_feats = (v == 256 || v == 224) ? v : 0;
+    g_tc_tile_feats = 0;
+    for (const auto& w : TC_WIDTHS) if (w.rows == v) g_tc_tile_feats = v;
     return old;
 }
 
@@ -1468,28 +1475,38 @@ static TcRows tc_rows(const TcExtra& ex) {
     return rs;
 }
 
-// Weight rows per tile of the token-lane persistent product of T tokens and N features: 256 in four stages, or 224 in
-// five.  A 64-deep k-step costs a tile about 600 cycles with four stages in flight whatever its width (the operands'
-// latency sets the pace, not their bytes) and about 500 with five (then issuing the step's products does); the narrower
-// tile wins where its count does not add a round over the SMs.
+// Weight rows per tile of the token-lane persistent product of T tokens and N features: the least time for the rounds of its
+// tiles over the SMs.
 static int tc_token_lane_rows(int T, int N) {
     if (g_tc_tile_feats) return g_tc_tile_feats;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int t_tiles = rb_ceil_div(T, 128);
-    const double c256 = 600.0 * rb_ceil_div((long long)rb_ceil_div(N, 256) * t_tiles, sms);
-    const double c224 = 500.0 * rb_ceil_div((long long)rb_ceil_div(N, 224) * t_tiles, sms);
-    return c224 < c256 ? 224 : 256;
+    const long long t_tiles = rb_ceil_div(T, 128);
+    int best = 256;
+    double least = 0.0;
+    for (const auto& w : TC_WIDTHS) {
+        const double cost = w.ns * rb_ceil_div(rb_ceil_div(N, w.rows) * t_tiles, sms);
+        if (least == 0.0 || cost < least) { least = cost; best = w.rows; }
+    }
+    return best;
 }
 
-// Products with few output features over many tokens: in tiles of 256 features they would leave most SMs idle, each of the few
-// CTAs walking the whole depth alone and finishing with an epilogue that nothing hides.  Tiles of 64 features in eight stages.
-static bool tc_few_features(int T, int N) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return !g_tc_tile_feats && 2LL * rb_ceil_div(N, 256) * rb_ceil_div(T, 128) <= sms;
+// The token-lane persistent product in tiles of that many weight rows.
+static int launch_tc_token_lanes(const void* X, const void* W, void* C, int T, int N, int K, long long ldx, long long ldw, long long ldc, int mode,
+                                 const TcRows& rs, cudaStream_t s) {
+    const int rows = tc_token_lane_rows(T, N);
+    CUtensorMap mw, mx;
+    if (rb_tensor_map_bf16(W, N, K, ldw, rows, &mw)) return -1;
+    if (rb_tensor_map_bf16(X, T, K, ldx, 128, &mx)) return -1;
+    switch (rows) {
+        case 64: return launch_tc_persistent<128, 8, 2, 64>(mw, mx, C, T, N, K, ldc, mode, s, TcHeads{}, rs);
+        case 144: return launch_tc_persistent<128, 6, 2, 144>(mw, mx, C, T, N, K, ldc, mode, s, TcHeads{}, rs);
+        case 160: return launch_tc_persistent<128, 6, 2, 160>(mw, mx, C, T, N, K, ldc, mode, s, TcHeads{}, rs);
+        case 192: return launch_tc_persistent<128, 5, 2, 192>(mw, mx, C, T, N, K, ldc, mode, s, TcHeads{}, rs);
+        case 224: return launch_tc_persistent<128, 5, 2, 224>(mw, mx, C, T, N, K, ldc, mode, s, TcHeads{}, rs);
+        default: return launch_tc_persistent<128, 4, 2, 256>(mw, mx, C, T, N, K, ldc, mode, s, TcHeads{}, rs);
+    }
 }
 
 // Whether a product over T tokens applies row factors (rows that lack their RMS factor) in its epilogue: the streaming
@@ -1541,14 +1558,7 @@ extern "C" int rb_gemm_bf16(const void* X, const void* W, void* C, int c_dtype, 
         // (stored results) or adds 16 bytes at a time where they live (added results), which keeps the one epilogue that
         // nothing hides, the last, short.  rb_set_gemm_token_lanes(0) runs the form with a feature per lane instead.
         const bool flip = g_tc_token_lanes != 0;
-        if (flip) {
-            const bool narrow = tc_token_lane_rows(T, N) == 224, few = tc_few_features(T, N);
-            if (rb_tensor_map_bf16(W, N, K, ldw, few ? 64 : narrow ? 224 : 256, &mw)) return -1;
-            if (rb_tensor_map_bf16(X, T, K, ldx, 128, &mx)) return -1;
-            if (few) return launch_tc_persistent<128, 8, 2, 64>(mw, mx, C, T, N, K, ldc, mode, s, TcHeads{}, tc_rows(ex));
-            if (narrow) return launch_tc_persistent<128, 5, 2, 224>(mw, mx, C, T, N, K, ldc, mode, s, TcHeads{}, tc_rows(ex));
-            return launch_tc_persistent<128, 4, 2, 256>(mw, mx, C, T, N, K, ldc, mode, s, TcHeads{}, tc_rows(ex));
-        }
+        if (flip) return launch_tc_token_lanes(X, W, C, T, N, K, ldx, ldw, ldc, mode, tc_rows(ex), s);
         if (row_sumsq) RB_REFUSE("gemm: row factors over %d tokens need the token-lane persistent product", T);
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
@@ -1605,14 +1615,7 @@ extern "C" int rb_gemm_bf16_act(const void* X, const void* W, void* C, int T, in
     if (rb_act_make(&ex.act, kind, scale, gates, gate_ld, ff, blocks, mul, mul_dtype, mul_ld, mul_row, N)) return -1;
     cudaStream_t s = (cudaStream_t)stream;
     CUtensorMap mw, mx;
-    if (T > 256) {
-        const bool narrow = tc_token_lane_rows(T, N) == 224, few = tc_few_features(T, N);
-        if (rb_tensor_map_bf16(W, N, K, ldw, few ? 64 : narrow ? 224 : 256, &mw)) return -1;
-        if (rb_tensor_map_bf16(X, T, K, ldx, 128, &mx)) return -1;
-        if (few) return launch_tc_persistent<128, 8, 2, 64>(mw, mx, C, T, N, K, ldc, 0, s, TcHeads{}, tc_rows(ex));
-        if (narrow) return launch_tc_persistent<128, 5, 2, 224>(mw, mx, C, T, N, K, ldc, 0, s, TcHeads{}, tc_rows(ex));
-        return launch_tc_persistent<128, 4, 2, 256>(mw, mx, C, T, N, K, ldc, 0, s, TcHeads{}, tc_rows(ex));
-    }
+    if (T > 256) return launch_tc_token_lanes(X, W, C, T, N, K, ldx, ldw, ldc, 0, tc_rows(ex), s);
     const int bn = tc_bn(T);
     if (rb_tensor_map_bf16(W, N, K, ldw, TC_BM, &mw)) return -1;
     if (rb_tensor_map_bf16(X, T, K, ldx, bn, &mx)) return -1;

@@ -51,7 +51,7 @@ def lib():
             # the gated pair over 65 .. 128 tokens: 1 the streaming kernel with a token per lane (default), 0 a feature per lane
             _lib.rb_set_gemm_gated_stream(int(os.environ["REINFER_B200_GEMM_GATED_STREAM"]))
         if os.environ.get("REINFER_B200_GEMM_TILE_ROWS"):
-            # prompt portions: 256 or 224 weight rows a tile; default chosen per product
+            # prompt portions: 256, 224, 192, 160, 144 or 64 weight rows a tile; default chosen per product
             _lib.rb_set_gemm_tile_features(int(os.environ["REINFER_B200_GEMM_TILE_ROWS"]))
         if os.environ.get("REINFER_B200_PDL", "1") == "0":
             _lib.rb_set_pdl(0)          # launch every kernel fully serialised (for comparisons)
@@ -851,9 +851,9 @@ def set_gemm_token_lanes(value: int) -> int:
 
 
 def set_gemm_tile_features(value: int) -> int:
-    """Weight rows per tile of the products over several token tiles (token-lane forms): 256 (four stages in
-    flight), 224 (five), or 0 = chosen per product by the rounds its tiles need over the SMs.  Returns the old
-    setting; for tests and comparisons."""
+    """Weight rows per tile of the products over several token tiles (token-lane forms): 256, 224, 192, 160, 144 or
+    64, or 0 = chosen per product by the rounds its tiles need over the SMs.  Returns the old setting; for tests and
+    comparisons."""
     return int(lib().rb_set_gemm_tile_features(c_int(int(value))))
 
 

@@ -77,6 +77,18 @@ def test_gemm_over_many_token_tiles_to_the_roundings_own_width(T, N, K, token_la
         ops.set_gemm_tile_features(old_feats)
 
 
+@pytest.mark.parametrize("T,N,K", [(257, 64, 64), (300, 288, 320), (385, 145, 136), (513, 320, 1024), (640, 2562, 72)])
+@pytest.mark.parametrize("rows", [64, 144, 160, 192])
+def test_gemm_tiles_of_every_width(T, N, K, rows):
+    """The token-lane product with each of the narrower tiles, at features that end inside a tile, on one and one past one."""
+    from reinfer_b200 import ops
+    old = ops.set_gemm_tile_features(rows)
+    try:
+        _many_token_tiles(ops, T, N, K)
+    finally:
+        ops.set_gemm_tile_features(old)
+
+
 def _many_token_tiles(ops, T, N, K):
     a = rnd(T, K, dtype=torch.bfloat16, seed=1)
     w = rnd(N, K, dtype=torch.bfloat16, scale=0.05, seed=2)
