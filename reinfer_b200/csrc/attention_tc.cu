@@ -691,6 +691,17 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
     }
 }
 
+template <int OPTIONS>
+static int fc_launch(dim3 grid, size_t smem, cudaStream_t s, const CUtensorMap& map, const FcArgs& a) {
+    static bool done = false;                          // once: the call costs the host some microseconds, as much as a launch
+    if (!done) {
+        const cudaError_t e = cudaFuncSetAttribute(fa_prefill_tc_kernel<OPTIONS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
+        done = true;
+    }
+    return rb_launch(fa_prefill_tc_kernel<OPTIONS>, grid, dim3(FC_THREADS), smem, s, map, a);
+}
+
 // q [T, QH, 128] bfloat16; cache: one layer's [num_pages, 2, KH, page_size, 128]; entries first_entry .. bring
 // cu_q[e+1] - cu_q[e] tokens each and hold kv_len[e] tokens after this step.  n_tiles: the sum over these
 // entries of ceil(tokens / (256 / Gc)), Gc = the largest of 16, 8, 4, 2, 1 that divides QH / KH.
@@ -728,11 +739,14 @@ extern "C" int rb_fa_prefill_tc(const void* q, const void* cache, long long num_
     static_assert(smem <= 232448, "more than the shared memory of an SM");
     if (n_tiles > 65535) RB_REFUSE("attention (tcgen05): %d row tiles in one launch", n_tiles);
     const int options = (softcap > 0.0f ? FC_CAP : 0) | (r1 ? FC_PENALTY : 0) | (bias ? FC_BIAS : 0);
-    auto kernel = options == 0 ? fa_prefill_tc_kernel<0> : options == FC_CAP ? fa_prefill_tc_kernel<FC_CAP> : options == FC_PENALTY ? fa_prefill_tc_kernel<FC_PENALTY> :
-        options == FC_BIAS ? fa_prefill_tc_kernel<FC_BIAS> : fa_prefill_tc_kernel<FC_CAP | FC_PENALTY | FC_BIAS>;
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
-    return rb_launch(kernel, dim3(KH * a.chunks, n_tiles), dim3(FC_THREADS), smem, (cudaStream_t)stream, map, a);
+    const dim3 grid(KH * a.chunks, n_tiles);
+    switch (options) {
+        case 0: return fc_launch<0>(grid, smem, (cudaStream_t)stream, map, a);
+        case FC_CAP: return fc_launch<FC_CAP>(grid, smem, (cudaStream_t)stream, map, a);
+        case FC_PENALTY: return fc_launch<FC_PENALTY>(grid, smem, (cudaStream_t)stream, map, a);
+        case FC_BIAS: return fc_launch<FC_BIAS>(grid, smem, (cudaStream_t)stream, map, a);
+        default: return fc_launch<FC_CAP | FC_PENALTY | FC_BIAS>(grid, smem, (cudaStream_t)stream, map, a);
+    }
 }
 
 // The group of query heads that share a CTA's rows, as rb_fa_prefill_tc chooses it, and the rows of a CTA (for the
