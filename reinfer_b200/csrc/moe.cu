@@ -240,6 +240,24 @@ __device__ __forceinline__ void moe_load8(const float* p, float (&v)[8]) {
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
+// The 32 sums of a warp's threads, sum i in lane i: in five rounds a lane hands half of what it still holds to its partner and adds
+// what comes back, 31 shuffles for all of them where a butterfly for each took 160.  Every sum's terms meet in the butterfly's
+// pairs: the same bits.  (2,048 tokens, 17 outputs of 2,048 columns: 26 -> 24 us; the rest is the rows' trips from L2.)
+__device__ __forceinline__ float moe_warp_sums(float (&v)[ROUTER_TOKENS][8], int lane) {
+    static_assert(ROUTER_TOKENS * 8 == 32, "a sum per lane");
+    float* f = &v[0][0];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool upper = lane & o;
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            const float keep = upper ? f[i + o] : f[i], give = upper ? f[i] : f[i + o];
+            f[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    return f[0];
+}
+
 template <typename TX, typename TW>
 __global__ void __launch_bounds__(ROUTER_THREADS)
 moe_router_kernel(const TX* __restrict__ x, const TW* __restrict__ w, const float* __restrict__ corr, float* __restrict__ gates,
@@ -287,13 +305,7 @@ moe_router_kernel(const TX* __restrict__ x, const TW* __restrict__ w, const floa
                 }
             }
         }
-#pragma unroll
-        for (int a = 0; a < ROUTER_TOKENS; ++a)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float v = warp_sum(acc[a][j]);
-                if (lane == 0) part[warp][a][j] = v;
-            }
+        (&part[warp][0][0])[lane] = moe_warp_sums(acc, lane);
         __syncthreads();
         if (threadIdx.x < ROUTER_TOKENS * 8) {
             const int a = threadIdx.x / 8, j = threadIdx.x % 8;
@@ -326,7 +338,14 @@ moe_router_cluster_kernel(const TX* __restrict__ x, const TW* __restrict__ w, co
     extern __shared__ float sm[];                              // per token: scores [n], choice [n], groups [n]
     __shared__ float part[ROUTER_THREADS / 32][ROUTER_TOKENS][8];
     asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-    pdl_trigger(); pdl_wait();
+    pdl_trigger();
+    {   // this CTA's rows of W do not come from the kernels before: they are called into L2 while those still run
+        const int per_cta = (n + ROUTER_CLUSTER - 1) / ROUTER_CLUSTER, first = blockIdx.x * per_cta;
+        const char* rows = reinterpret_cast<const char*>(w + (size_t)min(first, n) * h);
+        const size_t bytes = (size_t)max(min(per_cta, n - first), 0) * h * sizeof(TW);
+        for (size_t o = (size_t)threadIdx.x * 128; o < bytes; o += ROUTER_THREADS * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(rows + o));
+    }
+    pdl_wait();
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");    // every CTA of the cluster runs: its shared memory may be written
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = blockIdx.y * ROUTER_TOKENS, rank = blockIdx.x;
@@ -370,15 +389,7 @@ moe_router_cluster_kernel(const TX* __restrict__ x, const TW* __restrict__ w, co
                 }
             }
         }
-#pragma unroll
-        for (int a = 0; a < ROUTER_TOKENS; ++a)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (j < live) {                                // (uniform)
-                    const float v = warp_sum(acc[a][j]);
-                    if (lane == 0) part[warp][a][j] = v;
-                }
-            }
+        (&part[warp][0][0])[lane] = moe_warp_sums(acc, lane);
         __syncthreads();
         if (threadIdx.x < ROUTER_TOKENS * 8) {
             const int a = threadIdx.x / 8, j = threadIdx.x % 8;
