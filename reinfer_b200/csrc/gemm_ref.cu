@@ -88,9 +88,9 @@ static int gemm_ref_dispatch(const void* A, const void* W, void* C, int c_dtype,
 
 // ---- 32-bit operands that 16-byte copies can address -----------------------------------------------------------
 // K is cut into F32_SEGMENTS segments (each a multiple of F32_UNIT long, the last ones shorter or empty).  Within a segment
-// an output element is one chain of FMAs over ascending k from zero; the segments' sums are added in ascending order.  Both
-// kernels below do exactly that, so a token has the same bits whether one of them or the other computes it.
-// Both keep rows along K in shared memory ([row][steps of BK + 4] floats: with BK 16 or 32 eight rows' 16 bytes fall into
+// an output element is one chain of FMAs over ascending k from zero; the segments' sums are added in ascending order.  The
+// kernels below all do exactly that, so a token has the same bits whichever of them computes it.
+// The first two keep rows along K in shared memory ([row][steps of BK + 4] floats: with BK 16 or 32 eight rows' 16 bytes fall into
 // eight different groups of four banks), brought by cp.async; nothing is transposed: a thread reads four consecutive k of a
 // row at once.
 #define F32_UNIT 32
@@ -331,13 +331,25 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
     }
 }
 
+// Both forms of a kernel (store, add) may use that much dynamic shared memory.
+template <typename Kernel>
+static int f32_allow_shared(Kernel store, Kernel add, size_t bytes) {
+    cudaError_t e = cudaFuncSetAttribute(store, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(add, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return (int)e;
+}
+
 template <int BM, int BN, int TM, int TN, int STAGES>
 static int gemm_f32_tile(const float* A, const float* W, float* C, int accumulate, int M, int N, int K, long long lda,
                          long long ldw, long long ldc, cudaStream_t s) {
     using Tile = F32Tile<BM, BN, TM, TN, STAGES>;
     auto kernel = accumulate ? gemm_f32_tile_kernel<BM, BN, TM, TN, STAGES, 1> : gemm_f32_tile_kernel<BM, BN, TM, TN, STAGES, 0>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile::SMEM);
-    if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
+    static bool done = false;                                       // once: the calls cost the host as much as a launch
+    if (!done) {
+        if (int e = f32_allow_shared(gemm_f32_tile_kernel<BM, BN, TM, TN, STAGES, 0>, gemm_f32_tile_kernel<BM, BN, TM, TN, STAGES, 1>, Tile::SMEM)) return e;
+        done = true;
+    }
     return rb_launch(kernel, dim3(rb_ceil_div(M, BM), rb_ceil_div(N, BN)), dim3(Tile::THREADS), Tile::SMEM, s, A, W, C, M, N, K, lda, ldw, ldc);
 }
 
@@ -345,22 +357,139 @@ template <int TM>
 static int gemm_f32_few(const float* A, const float* W, float* C, int accumulate, int M, int N, int K, long long lda,
                         long long ldw, long long ldc, cudaStream_t s) {
     auto kernel = accumulate ? gemm_f32_few_kernel<TM, 1> : gemm_f32_few_kernel<TM, 0>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F32Few<TM>::SMEM);
-    if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
+    static bool done = false;                                       // once: the calls cost the host as much as a launch
+    if (!done) {
+        if (int e = f32_allow_shared(gemm_f32_few_kernel<TM, 0>, gemm_f32_few_kernel<TM, 1>, F32Few<TM>::SMEM)) return e;
+        done = true;
+    }
     return rb_launch(kernel, dim3(rb_ceil_div(N, 16), rb_ceil_div(M, 2 * TM)), dim3(F32_SEGMENTS * 32), F32Few<TM>::SMEM, s, A, W, C, M, N, K, lda, ldw, ldc);
 }
 
+// Many tokens, 128 x 128 outputs per CTA, 8 x 8 a thread.  Here the operands are transposed on the way in ([k][row], through
+// registers), so that a thread's 16 operands of one k are four loads of 16 bytes and its registers hold one k ahead, not four:
+// 64 sums, 32 operands and the next step's 16 numbers fit 128 registers, and two CTAs an SM.
+// 727 tokens over 19,456 x 2,560 weights 1.72 ms (42 TFLOP/s; the 64 x 128 tiles above 1.87), over 2,560 x 9,728 1.00 ms (1.11).
+#define F32W_ROW (128 + 4)
+template <int MODE>
+__global__ void __launch_bounds__(256, 2)
+gemm_f32_wide_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K,
+                     long long lda, long long ldw, long long ldc) {
+    constexpr int BK = 16;
+    extern __shared__ __align__(16) float f32_smem[];                // [2][A: BK rows of F32W_ROW, W: the same], then the running sums
+    float* run = f32_smem + 2 * 2 * BK * F32W_ROW + threadIdx.x;      // [64][256]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tx = (warp & 1) * 8 + (lane & 7), ty = (warp >> 1) * 4 + (lane >> 3);
+    const int m0 = blockIdx.x * 128, n0 = blockIdx.y * 128;
+    const int steps = (K + BK - 1) / BK, seg = f32_segment(K) / BK;
+    // a thread brings 16 bytes of rows r0 and r0 + 64 of either operand
+    const int r0 = threadIdx.x >> 2, c0 = (threadIdx.x & 3) * 4;
+    const float* ap = A + (size_t)(m0 + r0) * lda + c0;
+    const float* wp = W + (size_t)(n0 + r0) * ldw + c0;
+    float4 next[4];
+    auto fetch = [&](int step) {
+        const int k = step * BK;
+        const bool in = k + c0 < K;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        next[0] = in && m0 + r0 < M ? *reinterpret_cast<const float4*>(ap + k) : zero;
+        next[1] = in && m0 + r0 + 64 < M ? *reinterpret_cast<const float4*>(ap + 64 * lda + k) : zero;
+        next[2] = in && n0 + r0 < N ? __ldg(reinterpret_cast<const float4*>(wp + k)) : zero;
+        next[3] = in && n0 + r0 + 64 < N ? __ldg(reinterpret_cast<const float4*>(wp + 64 * ldw + k)) : zero;
+    };
+    auto put = [&](int buf) {
+        float* dst = f32_smem + buf * (2 * BK * F32W_ROW) + c0 * F32W_ROW + r0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float* d = dst + (i >> 1) * (BK * F32W_ROW) + (i & 1) * 64;
+            d[0] = next[i].x; d[F32W_ROW] = next[i].y; d[2 * F32W_ROW] = next[i].z; d[3 * F32W_ROW] = next[i].w;
+        }
+    };
+    pdl_trigger();
+    pdl_wait();
+    float acc[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
+    fetch(0);
+    put(0);
+    __syncthreads();
+#pragma unroll 1
+    for (int step = 0; step < steps; ++step) {
+        if (step + 1 < steps) fetch(step + 1);
+        if (step && step % seg == 0) {                              // a segment begins
+#pragma unroll
+            for (int i = 0; i < 64; ++i) {
+                float* r = run + i * 256;
+                *r = step == seg ? acc[i >> 3][i & 7] : *r + acc[i >> 3][i & 7];
+                acc[i >> 3][i & 7] = 0.0f;
+            }
+        }
+        const float* as = f32_smem + (step & 1) * (2 * BK * F32W_ROW) + ty * 4;
+        const float* ws = f32_smem + (step & 1) * (2 * BK * F32W_ROW) + BK * F32W_ROW + tx * 4;
+        float4 a[2][2], b[2][2];
+        a[0][0] = *reinterpret_cast<const float4*>(as); a[0][1] = *reinterpret_cast<const float4*>(as + 64);
+        b[0][0] = *reinterpret_cast<const float4*>(ws); b[0][1] = *reinterpret_cast<const float4*>(ws + 64);
+#pragma unroll
+        for (int k = 0; k < BK; ++k) {
+            if (k + 1 < BK) {
+                const float* an = as + (k + 1) * F32W_ROW;
+                const float* wn = ws + (k + 1) * F32W_ROW;
+                a[(k + 1) & 1][0] = *reinterpret_cast<const float4*>(an); a[(k + 1) & 1][1] = *reinterpret_cast<const float4*>(an + 64);
+                b[(k + 1) & 1][0] = *reinterpret_cast<const float4*>(wn); b[(k + 1) & 1][1] = *reinterpret_cast<const float4*>(wn + 64);
+            }
+            const float4 a0 = a[k & 1][0], a1 = a[k & 1][1], b0 = b[k & 1][0], b1 = b[k & 1][1];
+            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+        }
+        if (step + 1 < steps) put((step + 1) & 1);                  // (the buffer that was read in the step before)
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int gm = m0 + ty * 4 + (i & 3) + (i >> 2) * 64;
+        if (gm >= M) continue;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int gn = n0 + tx * 4 + (j & 3) + (j >> 2) * 64;
+            if (gn >= N) continue;
+            float sum = acc[i][j];
+            if (steps > seg) sum = run[(i * 8 + j) * 256] + sum;
+            float* c = C + (size_t)gm * ldc + gn;
+            *c = MODE == 0 ? sum : *c + sum;
+        }
+    }
+}
+
+static int gemm_f32_wide(const float* A, const float* W, float* C, int accumulate, int M, int N, int K, long long lda,
+                         long long ldw, long long ldc, cudaStream_t s) {
+    constexpr size_t smem = (2 * 2 * 16 * F32W_ROW + 64 * 256) * sizeof(float);
+    auto kernel = accumulate ? gemm_f32_wide_kernel<1> : gemm_f32_wide_kernel<0>;
+    static bool done = false;                                       // once: the calls cost the host as much as a launch
+    if (!done) {
+        if (int e = f32_allow_shared(gemm_f32_wide_kernel<0>, gemm_f32_wide_kernel<1>, smem)) return e;
+        done = true;
+    }
+    // (begun early, its CTAs would go where the kernel before leaves room, two to an SM beside idle ones)
+    return rb_launch_after(kernel, dim3(rb_ceil_div(M, 128), rb_ceil_div(N, 128)), dim3(256), smem, s, A, W, C, M, N, K, lda, ldw, ldc);
+}
+
 // Which kernel: up to 16 tokens the one for few (9 .. 16: its CTAs for the second eight find the weights in L2; 2,560 x 9,728
-// weights 2 x 53 us, 32 x 64 tiles 260 us).  Else the tile whose busiest SM is done first: a 64 x 128 tile takes an SM 80 units
-// (574 us at K = 9,728), a 32 x 64 tile 26, and 35 where it is alone on its SM.
+// weights 61 us, 32 x 64 tiles 260 us).  Else the tile whose busiest SM is done first: a 64 x 128 tile takes an SM 80 units
+// (574 us at K = 9,728), a 128 x 128 tile 134 (140 where it is alone on its SM), a 32 x 64 tile 26 (35).
 static int gemm_f32_dispatch(const float* A, const float* W, float* C, int accumulate, int M, int N, int K, long long lda,
                              long long ldw, long long ldc, cudaStream_t s) {
     if (M <= 2) return gemm_f32_few<1>(A, W, C, accumulate, M, N, K, lda, ldw, ldc, s);
     if (M <= 4) return gemm_f32_few<2>(A, W, C, accumulate, M, N, K, lda, ldw, ldc, s);
     if (M <= 16) return gemm_f32_few<4>(A, W, C, accumulate, M, N, K, lda, ldw, ldc, s);
-    const long long big = 80LL * rb_ceil_div((long long)rb_ceil_div(M, 64) * rb_ceil_div(N, 128), 148);
-    const long long mid = 26LL * rb_ceil_div((long long)rb_ceil_div(M, 32) * rb_ceil_div(N, 64), 148);
-    if ((mid > 35 ? mid : 35) < big) return gemm_f32_tile<32, 64, 4, 4, 4>(A, W, C, accumulate, M, N, K, lda, ldw, ldc, s);
+    auto busiest = [&](int bm, int bn) { return (long long)rb_ceil_div((long long)rb_ceil_div(M, bm) * rb_ceil_div(N, bn), 148); };
+    const long long wide = busiest(128, 128) == 1 ? 140 : 134 * busiest(128, 128);
+    const long long tile = 80 * busiest(64, 128);
+    const long long mid = busiest(32, 64) == 1 ? 35 : 26 * busiest(32, 64);
+    if (mid < tile && mid < wide) return gemm_f32_tile<32, 64, 4, 4, 4>(A, W, C, accumulate, M, N, K, lda, ldw, ldc, s);
+    if (wide < tile) return gemm_f32_wide(A, W, C, accumulate, M, N, K, lda, ldw, ldc, s);
     return gemm_f32_tile<64, 128, 8, 4, 3>(A, W, C, accumulate, M, N, K, lda, ldw, ldc, s);
 }
 

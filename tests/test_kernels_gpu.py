@@ -305,8 +305,8 @@ def test_gemm_plain(ta, tw, tc, T, N, K):
     assert torch.equal(c1[0], c[T // 2])
 
 
-@pytest.mark.parametrize("T", [1, 2, 3, 5, 8, 9, 16, 17, 33, 65, 129, 400])
-@pytest.mark.parametrize("N,K", [(1, 4), (15, 36), (17, 128), (65, 260), (129, 132), (300, 1000), (2700, 64)])
+@pytest.mark.parametrize("T", [1, 2, 3, 5, 8, 9, 16, 17, 33, 65, 129, 400, 650])
+@pytest.mark.parametrize("N,K", [(1, 4), (15, 36), (17, 128), (65, 260), (129, 132), (300, 1000), (2601, 64), (2600, 132)])
 def test_gemm_float32_tiles(T, N, K):
     """32-bit operands that 16-byte copies can address: every tile size at its edges (tokens, features, a last partial
     step along K), and the same bits for a token whatever else is in the batch.  Each result is the sum of
