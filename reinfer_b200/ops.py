@@ -680,10 +680,7 @@ def decode_splits(ctas: int, tiles: int, slots: int = DECODE_SLOTS, head_dim: in
         have finished; what is left streams at the memory bandwidth, less what the CTAs' fill and drain cost,
         which weighs the more the fewer tiles a CTA walks:   bytes left / 6.5 TB/s * (1 + 2.7 / tiles per CTA)
       - a CTA alone streams a 64-key tile of 128-wide heads in about a microsecond and needs about five to start
-        and finish; the kernel lasts as long as the CTA with most tiles:   (most tiles per CTA - 3) * 1 us + 5 us,
-        where contexts are short (up to eight tiles) plus 1.4 us for its second and its third tile, which have landed by
-        then but are worked on one after the other (the 8B shape: one request with three tiles 3.11 ms a step unsplit and
-        3.00 split in four, four requests of up to four tiles 3.09 and 2.99; with two tiles no difference)
+        and finish; the kernel lasts as long as the CTA with most tiles:   (most tiles per CTA - 3) * 1 us + 5 us
         (requests of unequal lengths: the longest alone decides this term, so splitting pays although the
         CTAs then come in several waves)
       - the larger of the two counts, plus the merge: about 2 us inside a cluster (up to 16 splits, all CTAs
@@ -715,8 +712,6 @@ def decode_splits(ctas: int, tiles: int, slots: int = DECODE_SLOTS, head_dim: in
         early = min(total_tiles, min(ctas * n, slots) * ahead)
         t_bw = (total_tiles - early) * tile_bw_us * (1.0 + 2.7 / per_avg)
         t_lat = max(0, per - ahead) * tile_us + 5.0
-        if tiles <= 8:
-            t_lat += 1.4 * (min(per, ahead) - 1)
         if n == 1:
             merge = 0.0
         elif n <= min(MAX_CLUSTER_SPLITS, head_dim) and ATTN_CLUSTER_MERGE and \

@@ -87,6 +87,12 @@ def test_decode_splits_model():
     assert decode_splits(32 * 8, 67, total_tiles=32 * 8 * 36) == 2
     # wider heads: the same decisions at the same number of bytes
     assert decode_splits(64 * 8, 64, head_dim=256) == 1
+    # a context that grows by a tile at a time asks for few plans (a captured step is made for each) and for none that shares
+    # its keys out among a CTA a tile and takes that back at the next
+    for pairs in (1, 8, 16, 32, 64, 128):
+        plans = [decode_splits(pairs, t) for t in range(1, 25)]
+        assert plans[:3] == [1, 1, 1] and len(set(plans[:9])) <= 3, plans
+        assert all(abs(b - a) <= 1 for a, b in zip(plans, plans[1:])), plans
 
 
 def test_sampling_params_checks():
