@@ -275,11 +275,17 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
             if (r0 + 4 * i < 2 * TM) cp_async16(dst(s) + (uint32_t)((16 + 4 * i) * F32_ROW) * 4u, real ? ap + (size_t)(4 * i) * lda + s * F32_UNIT : A, real);
         }
     };
-    // the weights do not come from the kernels before: their first tiles are asked for before those have ended
+    // The first tiles of W are called into L2 while the kernels before still run, and read behind the wait: one of those may be
+    // making W.
     pdl_trigger();
 #pragma unroll 1
-    for (int s = 0; s < STAGES - 1 && s < steps; ++s) load_w(s);
+    for (int i = lane; i < 16 * (STAGES - 1); i += 32) {
+        const int row = n0 + (i & 15), s = i >> 4;
+        if (row < N && s < steps) asm volatile("prefetch.global.L2 [%0];" ::"l"(W + (size_t)row * ldw + (first + s) * F32_UNIT));
+    }
     pdl_wait();
+#pragma unroll 1
+    for (int s = 0; s < STAGES - 1 && s < steps; ++s) load_w(s);
 #pragma unroll 1
     for (int s = 0; s < STAGES - 1; ++s) {
         if (s < steps) load_a(s);

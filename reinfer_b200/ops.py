@@ -316,7 +316,7 @@ def swiglu(gu: torch.Tensor, out: torch.Tensor) -> None:
 
 
 def gemm_ref(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, accumulate: bool = False) -> None:
-    """c[M,N] (=|+=) a[M,K] @ w[N,K]^T on the CUDA cores in 32-bit."""
+    """c[M,N] (=|+=) a[M,K] @ w[N,K]^T on the CUDA cores in 32-bit.  Both operands may come from the kernel launched before."""
     M, K = a.shape
     N = w.shape[0]
     _need(w.shape[1] == K and tuple(c.shape) == (M, N), "gemm: shapes")
@@ -861,7 +861,9 @@ def gemm_bf16(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, accumulate: boo
               row_scale=None) -> None:
     """c[T,N] (=|+=) a[T,K] @ w[N,K]^T on the tensor cores (tcgen05, TMA); bf16 operands, float
     accumulation, c bfloat16 or float32.  Operands that TMA cannot address (a row stride that is no
-    multiple of 8 elements, a base that is not 16-byte aligned) go to the plain kernel instead."""
+    multiple of 8 elements, a base that is not 16-byte aligned) go to the plain kernel instead.  w is a weight: a bfloat16
+    product over up to 256 tokens - this one and the others below - fetches its first tiles while the kernel of this library in front of it
+    still runs, so w must be complete when that kernel starts."""
     global _gemm_ws
     T, K = a.shape
     N = w.shape[0]

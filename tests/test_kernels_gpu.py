@@ -329,6 +329,25 @@ def test_gemm_float32_tiles(T, N, K):
             assert torch.equal(part, c[t:t + n])
 
 
+@pytest.mark.parametrize("T", [1, 4, 8, 16, 40, 650])
+def test_gemm_float32_of_a_matrix_the_kernel_before_makes(T):
+    """W is the result of a product right in front on the same stream, another one every time: what is read is what that product
+    left, the bits that come out once it has long ended."""
+    from reinfer_b200 import ops
+    N, K = 4096, 1024
+    x, q = rnd(T, K, dtype=torch.float32, seed=1), rnd(K, 64, dtype=torch.float32, seed=2)
+    w = torch.zeros(N, K, device=DEV)
+    for k in range(6):
+        p = rnd(N, 64, dtype=torch.float32, seed=10 + k)
+        c, again = torch.full((T, N), math.nan, device=DEV), torch.full((T, N), math.nan, device=DEV)
+        torch.cuda.synchronize()
+        ops.gemm_ref(p, q, w)
+        ops.gemm_ref(x, w, c)
+        torch.cuda.synchronize()
+        ops.gemm_ref(x, w, again)
+        assert torch.equal(c, again), k
+
+
 @pytest.mark.parametrize("h,rows", [(64, 1), (96, 5), (1000, 3), (4096, 2), (5120, 4)])
 @pytest.mark.parametrize("out_dtype,w_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16),
                                                (torch.bfloat16, torch.float32)])
