@@ -247,10 +247,10 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
     constexpr int STAGES = Few::STAGES;
     extern __shared__ __align__(16) float f32_smem[];
     __shared__ float sums[F32_SEGMENTS][2 * TM][16];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n0 = blockIdx.x * 16;
-    A += (size_t)blockIdx.y * (2 * TM) * lda;                       // this CTA's tokens
-    C += (size_t)blockIdx.y * (2 * TM) * ldc;
-    M = min(M - (int)blockIdx.y * 2 * TM, 2 * TM);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n0 = blockIdx.y * 16;
+    A += (size_t)blockIdx.x * (2 * TM) * lda;                       // this CTA's tokens: CTAs of the same weights are neighbours
+    C += (size_t)blockIdx.x * (2 * TM) * ldc;
+    M = min(M - (int)blockIdx.x * 2 * TM, 2 * TM);
     const int all = (K + F32_UNIT - 1) / F32_UNIT, seg = f32_segment(K) / F32_UNIT;
     const int first = min(warp * seg, all), steps = min(seg, all - first);
     const float* own = f32_smem + (size_t)warp * STAGES * Few::STAGE_FLOATS;
@@ -368,7 +368,7 @@ static int gemm_f32_few(const float* A, const float* W, float* C, int accumulate
         if (int e = f32_allow_shared(gemm_f32_few_kernel<TM, 0>, gemm_f32_few_kernel<TM, 1>, F32Few<TM>::SMEM)) return e;
         done = true;
     }
-    return rb_launch(kernel, dim3(rb_ceil_div(N, 16), rb_ceil_div(M, 2 * TM)), dim3(F32_SEGMENTS * 32), F32Few<TM>::SMEM, s, A, W, C, M, N, K, lda, ldw, ldc);
+    return rb_launch(kernel, dim3(rb_ceil_div(M, 2 * TM), rb_ceil_div(N, 16)), dim3(F32_SEGMENTS * 32), F32Few<TM>::SMEM, s, A, W, C, M, N, K, lda, ldw, ldc);
 }
 
 // Many tokens, 128 x 128 outputs per CTA, 8 x 8 a thread.  Here the operands are transposed on the way in ([k][row], through
@@ -482,8 +482,9 @@ static int gemm_f32_wide(const float* A, const float* W, float* C, int accumulat
     return rb_launch_after(kernel, dim3(rb_ceil_div(M, 128), rb_ceil_div(N, 128)), dim3(256), smem, s, A, W, C, M, N, K, lda, ldw, ldc);
 }
 
-// Which kernel: up to 16 tokens the one for few (9 .. 16: its CTAs for the second eight find the weights in L2; 2,560 x 9,728
-// weights 61 us, 32 x 64 tiles 260 us).  Else the tile whose busiest SM is done first: a 64 x 128 tile takes an SM 80 units
+// Which kernel: up to 16 tokens the one for few (2,560 x 9,728 weights, 16 tokens: 67 us, 32 x 64 tiles 260 us; 9 .. 16 tokens are
+// two CTAs a weight, neighbours in the grid, so that the second finds it in L2 however large W is: 16 tokens over 19,456 x 2,560
+// weights 82 us, 89 with the second eight behind all of W; over 151,936 x 2,560 676 and 687).  Else the tile whose busiest SM is done first: a 64 x 128 tile takes an SM 80 units
 // (574 us at K = 9,728), a 128 x 128 tile 134 (140 where it is alone on its SM), a 32 x 64 tile 26 (35).
 static int gemm_f32_dispatch(const float* A, const float* W, float* C, int accumulate, int M, int N, int K, long long lda,
                              long long ldw, long long ldc, cudaStream_t s) {
