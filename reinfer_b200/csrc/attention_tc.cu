@@ -333,44 +333,40 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
         // the scores of two tiles before are there, a tile ahead of their use; values wait for the product of the tile
         // before, and are needed half a tile after its rows began.  (One ring of six slots in the order of use had the
         // keys wait for that product too: the rows then waited 800 of 4,700 cycles for their scores.)
-        // Block-table entries 32 at a time.
+        // Block-table entries 32 at a time, in windows that begin at multiples of 32, which a half's pages (eight at most) never
+        // cross: the window of the keys, the one before it (values lie up to 24 pages behind the keys that went out before them), and
+        // the one after it, asked for a window ahead of its use.
         const int box_keys = min(a.page_size, FC_BN);              // keys that one request brings
         const int subs = FC_BN / box_keys;
-        const uint32_t lead = lane == 0 ? 1u : 0u;                 // every lane waits, lane 0's requests take effect
-        int cached_first = 0, cached = -1;
-        bool have = false, ok = true;
+        const uint32_t lead = lane == 0 ? 1u : 0u;
+        auto entries = [&](int w) { return w * 32 + lane < a.max_pages ? bt[w * 32 + lane] : -1; };
+        int window = ((t_begin * FC_BN) >> a.page_shift) >> 5;
+        int before = -1, here = entries(window), after = entries(window + 1);
+        bool ok = true;
         for (int step = 0; step < 2 * n_tiles + 1 && ok; ++step) { // keys 0; keys 1, values 0; keys 2, values 1; ...
             const int values = step > 0 && !(step & 1), tile = values ? step / 2 - 1 : (step + 1) / 2;
             if (tile >= n_tiles) continue;
 #pragma unroll 1
             for (int half = 2 * tile; half < min(2 * tile + 2, n_halves); ++half) {
                 const int k0 = (t_begin + half) * FC_BN;
-                const int pi0 = k0 >> a.page_shift;
-                const int need_last = (k0 + (subs - 1) * box_keys) >> a.page_shift;
-                if (!have || need_last >= cached_first + 32 || pi0 < cached_first) {
-                    // (values lie up to 192 keys behind the keys that went out before them: 24 pages at most, and a half has 8)
-                    cached_first = max(pi0 - ((3 * FC_BN + a.page_size - 1) >> a.page_shift), 0);
-                    cached = (cached_first + lane < a.max_pages) ? bt[cached_first + lane] : -1;
-                    have = true;
-                }
+                const int own = (k0 >> a.page_shift) >> 5;         // (a half is at most eight pages behind the last: one window further)
+                if (own > window) { before = here; here = after; after = entries(++window + 1); }
                 const int s = values ? FC_VSLOT(half) : FC_KSLOT(tile) + (half & 1), use = values ? tile : tile >> 1;
-                { FC_T0(); if (use && !fc_wait(smem_u32(&sh->empty[s]), (uint32_t)((use & 1) ^ 1), abort_flag, 11)) { ok = false; break; } FC_ADD(0); }
-                FC_T0();
                 const uint32_t full = smem_u32(&sh->full[s]);
                 const uint32_t dst0 = stages_u + s * FC_KV_BYTES;
-                // pages of this half that hold keys: a lane each, then one request a page
+                // A lane for each page of this half, which makes the page's request itself, all in one instruction.  (Lane 0 making them
+                // one after the other took some 200 cycles a request: 16 of them per 64 keys and values in pages of 8 keys are more than
+                // the 2,000 that the products and rows need.  32 query over 8 kv heads, 2,048 tokens behind 14,336 others:
+                // pages of 8 keys 951 -> 618 us, of 16 652 -> 526, of 64 531 -> 525.)
                 const int my_key = k0 + lane * box_keys;
-                const int my_page = __shfl_sync(0xffffffffu, cached, ((my_key >> a.page_shift) - cached_first) & 31);
+                const int my_page = __shfl_sync(0xffffffffu, own == window ? here : before, (my_key >> a.page_shift) & 31);
                 const uint32_t there = __ballot_sync(0xffffffffu, lane < subs && my_key < kv_end && my_page >= 0);
+                const int my_index = (my_page * 2 + values) * a.KH + kh, grp = (k0 & (a.page_size - 1)) >> 3;
+                { FC_T0(); if (use && !fc_wait(smem_u32(&sh->empty[s]), (uint32_t)((use & 1) ^ 1), abort_flag, 11)) { ok = false; break; } FC_ADD(0); }
+                FC_T0();
                 mbar_expect_tx_lead(full, (uint32_t)(__popc(there) * box_keys * 256), lead);
-#pragma unroll 1
-                for (int u = 0; u < subs; ++u) {
-                    const int page = __shfl_sync(0xffffffffu, my_page, u);
-                    if (!((there >> u) & 1u)) continue;
-                    const int key = k0 + u * box_keys;
-                    const int grp = (key & (a.page_size - 1)) >> 3;          // first 8-key group inside the page
-                    tma_load_5d_lead(dst0 + (uint32_t)(u * (box_keys >> 3) * FC_GROUP), &map_kv, 0, 0, 0, grp, (page * 2 + values) * a.KH + kh, full, lead);
-                }
+                __syncwarp();                                      // the barrier expects the bytes before the first of them can arrive
+                tma_load_5d_lead(dst0 + (uint32_t)((lane & 7) * (box_keys >> 3) * FC_GROUP), &map_kv, 0, 0, 0, grp, my_index, full, (there >> lane) & 1u);
                 if (lead) sh->uses[s] = use + 1;
                 FC_ADD(1);
             }

@@ -716,6 +716,73 @@ def test_prompt_attention_ends_anywhere_in_a_tile(QH, KH, lens, q_lens):
     assert ops.kernel_error() == 0
 
 
+def prompt_attention_setup(lens, q_lens, QH, KH, page, seed):
+    """Requests on shuffled pages of 128-wide heads; what no request holds is NaN."""
+    d, g = 128, torch.Generator(device=DEV).manual_seed(seed)
+    pages = [-(-n // page) for n in lens]
+    ids = torch.randperm(sum(pages) + 3, generator=torch.Generator().manual_seed(seed)).to(torch.int32)
+    cache = torch.full((sum(pages) + 3, 2, KH, page, d), math.nan, dtype=torch.bfloat16, device=DEV)
+    bt = torch.full((len(lens), max(pages) + 1), -1, dtype=torch.int32)
+    kv = []
+    for r, n in enumerate(lens):
+        held = ids[sum(pages[:r]):sum(pages[:r + 1])]
+        bt[r, :pages[r]] = held
+        kv.append(torch.randn(n, 2, KH, d, generator=g, device=DEV).to(torch.bfloat16))
+        at = torch.arange(n, device=DEV)
+        cache[held.to(DEV).long()[at // page], :, :, at % page] = kv[-1]
+    q = (1.5 * torch.randn(sum(q_lens), QH, d, generator=g, device=DEV)).to(torch.bfloat16)
+    return q, cache, bt, kv
+
+
+def prompt_attention_truth(q, kv, q_lens, scale, window=0, chunk=0, softcap=0.0, penalty=None, bias=None, sink=None, gate=None):
+    out, t0 = torch.zeros(q.shape, dtype=torch.float64, device=DEV), 0
+    for x, n in zip(kv, q_lens):
+        i, j = torch.arange(x.shape[0] - n, x.shape[0], device=DEV)[:, None], torch.arange(x.shape[0], device=DEV)
+        dist = (i - j).clamp(min=0)
+        seen = j <= i
+        if window:
+            seen &= i - j < window
+        if chunk:
+            seen &= i // chunk == j // chunk
+        for h in range(q.shape[1]):
+            k, v = x[:, 0, h * x.shape[2] // q.shape[1]].double(), x[:, 1, h * x.shape[2] // q.shape[1]].double()
+            s = q[t0:t0 + n, h].double() @ k.t() * scale
+            if softcap:
+                s = softcap * torch.tanh(s / softcap)
+            if penalty is not None:
+                s = s - penalty[0][h].double() * torch.log1p(penalty[1][h].double() * dist)
+            if bias is not None:
+                s = s + bias[h].double()[dist.clamp(max=bias.shape[1] - 1)]
+            s = s.masked_fill(~seen, -math.inf)
+            if sink is not None:
+                s = torch.cat([s, sink[h].double().expand(n, 1)], dim=1)
+            out[t0:t0 + n, h] = torch.softmax(s, dim=1)[:, :x.shape[0]] @ v
+        t0 += n
+    return out if gate is None else out * torch.sigmoid(gate.double()).view(out.shape)
+
+
+@pytest.mark.parametrize("page", [8, 16, 32, 64, 128])
+@pytest.mark.parametrize("window", [0, 300])
+def test_prompt_attention_over_pages_of_every_size(page, window):
+    """The tcgen05 attention over block tables of many and of few entries (its producer holds 32 at a time), with pages before the window
+    given back, against 64-bit sums.  P and the result are rounded to bfloat16: three half units of 2^-8 of the largest value."""
+    from reinfer_b200 import ops
+    QH, KH, lens, q_lens = 8, 2, [1985, 833, 64], [600, 833, 40]
+    q, cache, bt, kv = prompt_attention_setup(lens, q_lens, QH, KH, page, 11 + page)
+    if window:
+        for r, (n, m) in enumerate(zip(lens, q_lens)):
+            first = max(0, n - m - window + 1) // page
+            cache[bt[r, :first].to(DEV).long()] = math.nan
+            bt[r, :first] = -1
+    as_int = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    out = torch.full_like(q, math.nan)
+    ops.fa_prefill_tc(q, cache, bt.to(DEV), as_int([sum(q_lens[:r]) for r in range(len(lens) + 1)]), as_int(lens), out, 0, len(lens), q_lens,
+                      QH, KH, 128, page, window, 128 ** -0.5)
+    ref = prompt_attention_truth(q, kv, q_lens, 128 ** -0.5, window=window)
+    assert (out.double() - ref).abs().max().item() <= 3 * 2.0 ** -9 * max(x[:, 1].float().abs().max().item() for x in kv)
+    assert ops.kernel_error() == 0
+
+
 def test_attention_finds_one_far_key():
     """One key among hundreds gets a score that stands out; the output must be its value."""
     from reinfer_b200 import ops
