@@ -134,8 +134,6 @@ paged_attention_ref_kernel(const TA* __restrict__ q, const TC* __restrict__ cach
 // Bound by latency: a block's 32 scores are one chain of d loads and FMAs per lane.  727 tokens in four prompts of 40 to 300, 32
 // query over 8 kv heads of 128, 32 bits: the prompts and seven decode steps of four requests take 68 us a
 // launch on average, with the kernel above 493.
-#define RP_WARPS 8
-
 template <typename T> __device__ __forceinline__ float4 load4(const T* p);
 template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
 template <> __device__ __forceinline__ float4 load4<bf16>(const bf16* p) {
@@ -144,8 +142,8 @@ template <> __device__ __forceinline__ float4 load4<bf16>(const bf16* p) {
 }
 
 // G query heads of one kv head per CTA, value heads of at most 128 * NV numbers (G * NV <= 4).
-template <typename TA, typename TC, int G, int NV>
-__global__ void __launch_bounds__(RP_WARPS * 32)
+template <typename TA, typename TC, int G, int NV, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
 paged_attention_split_kernel(const TA* __restrict__ q, const TC* __restrict__ cache,
                              const int* __restrict__ block_table, const int* __restrict__ tok_row,
                              const int* __restrict__ positions, TA* __restrict__ out,
@@ -155,15 +153,15 @@ paged_attention_split_kernel(const TA* __restrict__ q, const TC* __restrict__ ca
                              int v_in_k, const float* __restrict__ gate, long long gate_stride) {
     pdl_trigger(); pdl_wait();
     extern __shared__ __align__(16) float rp_smem[];
-    __shared__ __align__(16) float ps[RP_WARPS][32][G];
-    __shared__ const TC* rows[RP_WARPS][32];
-    __shared__ float ms[RP_WARPS][G], ls[RP_WARPS][G];
+    __shared__ __align__(16) float ps[WARPS][32][G];
+    __shared__ const TC* rows[WARPS][32];
+    __shared__ float ms[WARPS][G], ls[WARPS][G];
     float* qs = rp_smem;                                       // [G][d]
-    float* parts = rp_smem + G * d;                            // [RP_WARPS][G][dv]
+    float* parts = rp_smem + G * d;                            // [WARPS][G][dv]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x, hq0 = blockIdx.y * G;
     const TA* qp = q + ((size_t)t * QH + hq0) * d;
-    for (int i = threadIdx.x; i < G * d; i += RP_WARPS * 32) qs[i] = to_f32(qp[i]);
+    for (int i = threadIdx.x; i < G * d; i += WARPS * 32) qs[i] = to_f32(qp[i]);
     __syncthreads();
     const int kh = hq0 / (QH / KH);
     const int pos = positions[t];
@@ -185,7 +183,7 @@ paged_attention_split_kernel(const TA* __restrict__ q, const TC* __restrict__ ca
 #pragma unroll
         for (int n = 0; n < NV; ++n) acc[g][n] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    for (int b = lo / 32 + ((warp - lo / 32) & (RP_WARPS - 1)); b * 32 <= pos; b += RP_WARPS) {
+    for (int b = lo / 32 + ((warp - lo / 32) & (WARPS - 1)); b * 32 <= pos; b += WARPS) {
         const int key = b * 32 + lane;
         bool valid = key >= lo && key <= pos;
         const int page = (valid && key / page_size < max_pages) ? bt[key / page_size] : -1;
@@ -264,14 +262,14 @@ paged_attention_split_kernel(const TA* __restrict__ q, const TC* __restrict__ ca
         }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < G * dv; i += RP_WARPS * 32) {
+    for (int i = threadIdx.x; i < G * dv; i += WARPS * 32) {
         const int g = i / dv, dim = i - g * dv, hq = hq0 + g;
         float top = sink ? sink[hq] : -INFINITY;
 #pragma unroll
-        for (int w = 0; w < RP_WARPS; ++w) top = fmaxf(top, ms[w][g]);
+        for (int w = 0; w < WARPS; ++w) top = fmaxf(top, ms[w][g]);
         float sum = 0.0f, val = 0.0f;
 #pragma unroll
-        for (int w = 0; w < RP_WARPS; ++w) {
+        for (int w = 0; w < WARPS; ++w) {
             const float f = ms[w][g] == -INFINITY ? 0.0f : expf(ms[w][g] - top);
             sum += f * ls[w][g];
             val += f * parts[(size_t)(w * G + g) * dv + dim];
@@ -305,17 +303,26 @@ extern "C" int rb_paged_attention_ref(const void* q, const void* cache, int dtyp
     cudaStream_t s = (cudaStream_t)stream;
     if (dtype != RB_F32 && dtype != RB_BF16) RB_REFUSE("attention: dtype %d", dtype);
     // rows of four numbers at a time: a rule on sizes and alignment only, so that a token takes the same kernel under every cut
-    if (d % 4 == 0 && dv % 4 == 0 && ((uintptr_t)cache & (dtype == RB_F32 ? 15 : 7)) == 0) {
-        const int group = QH / KH, most = 512 / ((dv + 127) / 128 * 128);
-        const int G = group % 4 == 0 && most >= 4 ? 4 : group % 2 == 0 && most >= 2 ? 2 : 1;
-        const size_t smem = (size_t)(G * d + RP_WARPS * G * dv) * sizeof(float);
+    const int group = QH / KH, most = 512 / ((dv + 127) / 128 * 128);
+    const int G = group % 4 == 0 && most >= 4 ? 4 : group % 2 == 0 && most >= 2 ? 2 : 1;
+    if (d % 4 == 0 && dv % 4 == 0 && ((uintptr_t)cache & (dtype == RB_F32 ? 15 : 7)) == 0 && QH / G <= 65535) {
+        // How many warps share a token's keys: as there can be 32-key blocks in a chunk or a window.  Eight of which most find nothing
+        // still start, and are merged (2,047 tokens, 5 heads of 80, chunks of 64 keys, 16 bits: 165 us with eight warps, 65 with two,
+        // one warp a head as in the kernel at the top 92).
+        int blocks = 8;
+        if (chunk > 0) blocks = min(blocks, chunk % 32 ? chunk / 32 + 2 : chunk / 32);
+        if (window > 0 && window < 256) blocks = min(blocks, (window + 30) / 32 + 1);
+        const int warps = blocks <= 3 ? 2 : blocks <= 6 ? 4 : 8;
+        const size_t smem = (size_t)(G * d + warps * G * dv) * sizeof(float);
         const dim3 grid(n_tokens, QH / G);
-#define RP_LAUNCH(TT, GG) rb_launch(paged_attention_split_kernel<TT, TT, GG, 4 / GG>, grid, dim3(RP_WARPS * 32), smem, s, \
+#define RP_LAUNCH(TT, GG) (warps == 2 ? RP_LAUNCH_W(TT, GG, 2) : warps == 4 ? RP_LAUNCH_W(TT, GG, 4) : RP_LAUNCH_W(TT, GG, 8))
+#define RP_LAUNCH_W(TT, GG, WW) rb_launch(paged_attention_split_kernel<TT, TT, GG, 4 / GG, WW>, grid, dim3(WW * 32), smem, s, \
             (const TT*)q, (const TT*)cache, block_table, tok_row, positions, (TT*)out, QH, KH, d, dv, page_size, max_pages, window, scale, \
             chunk, r1, r2, out_scale, bias, bias_rows, softcap, sink, v_in_k, gate, gate_stride)
         if (dtype == RB_F32) return G == 4 ? RP_LAUNCH(float, 4) : G == 2 ? RP_LAUNCH(float, 2) : RP_LAUNCH(float, 1);
         return G == 4 ? RP_LAUNCH(bf16, 4) : G == 2 ? RP_LAUNCH(bf16, 2) : RP_LAUNCH(bf16, 1);
 #undef RP_LAUNCH
+#undef RP_LAUNCH_W
     }
     dim3 grid(n_tokens, rb_ceil_div(QH, RA_WARPS));
     const size_t smem = (size_t)RA_WARPS * d * sizeof(float);

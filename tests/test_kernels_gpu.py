@@ -716,6 +716,29 @@ def test_prompt_attention_ends_anywhere_in_a_tile(QH, KH, lens, q_lens):
     assert ops.kernel_error() == 0
 
 
+@pytest.mark.parametrize("QH,KH,d", [(4, 1, 32), (6, 3, 96), (5, 5, 80)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("window,chunk", [(1, 0), (2, 0), (33, 0), (34, 0), (65, 0), (66, 0), (161, 0), (162, 0), (0, 32), (0, 33), (0, 64), (0, 65), (0, 160),
+                                          (0, 192), (0, 193), (70, 128)])
+def test_paged_attention_plain_over_short_masks(QH, KH, d, dtype, window, chunk):
+    """Windows and chunks on both sides of the sizes at which fewer warps share a token's keys; and a token's bits do not depend on
+    the tokens beside it."""
+    from reinfer_b200 import ops
+    lens, q_lens = [1, 37, 64, 131, 400], [1, 5, 64, 131, 330]
+    s = paged_setup(lens, q_lens, QH, KH, d, 16, dtype)
+    out, scale = torch.full_like(s["q"], math.nan), d ** -0.5
+    ops.paged_attention_ref(s["q"], s["cache"], s["bt"], s["tok_row"], s["positions"], out, QH, KH, d, 16, window, scale, chunk=chunk)
+    kv = [torch.stack([k, v], dim=1).to(DEV) for k, v in zip(s["ks"], s["vs"])]
+    ref = prompt_attention_truth(s["q"], kv, q_lens, scale, window=window, chunk=chunk)
+    tol = 1.5e-2 if dtype == torch.bfloat16 else 1e-5
+    assert (out.double() - ref).abs().max().item() <= tol * ref.abs().max().item()
+    for t in (0, 7, 190, 530):
+        one = torch.full_like(out[t:t + 1], math.nan)
+        ops.paged_attention_ref(s["q"][t:t + 1], s["cache"], s["bt"], s["tok_row"][t:t + 1], s["positions"][t:t + 1], one, QH, KH, d, 16, window,
+                                scale, chunk=chunk)
+        assert torch.equal(one, out[t:t + 1])
+
+
 def prompt_attention_setup(lens, q_lens, QH, KH, page, seed):
     """Requests on shuffled pages of 128-wide heads; what no request holds is NaN."""
     d, g = 128, torch.Generator(device=DEV).manual_seed(seed)
