@@ -1475,14 +1475,18 @@ static TcRows tc_rows(const TcExtra& ex) {
     return rs;
 }
 
-// Weight rows per tile of the token-lane persistent product of T tokens and N features: the least time for the rounds of its
-// tiles over the SMs.
-static int tc_token_lane_rows(int T, int N) {
+// Weight rows per tile of the token-lane persistent product of T tokens, N features and depth K: the least time for the rounds of
+// its tiles over the SMs.  Up to three k-steps a tile's set-up and epilogue are most of it, which two rounds of tiles of 64 hide
+// better than one of wider ones does: 400 tokens, 2,560 features, K = 64 4.8 us in tiles of 64 and 5.3 of 144; 1,024 tokens, 1,536
+// features, K = 128 5.5 and 6.0; from K = 512 on one round of 144 is the faster.
+#define TC_SHALLOW (3 * TC_BK)
+static int tc_token_lane_rows(int T, int N, int K) {
     if (g_tc_tile_feats) return g_tc_tile_feats;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long long t_tiles = rb_ceil_div(T, 128);
+    if (K <= TC_SHALLOW && 2 * rb_ceil_div(N, 256) * t_tiles <= sms) return 64;
     int best = 256;
     double least = 0.0;
     for (const auto& w : TC_WIDTHS) {
@@ -1492,10 +1496,13 @@ static int tc_token_lane_rows(int T, int N) {
     return best;
 }
 
+// The same, for tests and tuning.
+extern "C" int rb_gemm_token_lane_rows(int T, int N, int K) { return tc_token_lane_rows(T, N, K); }
+
 // The token-lane persistent product in tiles of that many weight rows.
 static int launch_tc_token_lanes(const void* X, const void* W, void* C, int T, int N, int K, long long ldx, long long ldw, long long ldc, int mode,
                                  const TcRows& rs, cudaStream_t s) {
-    const int rows = tc_token_lane_rows(T, N);
+    const int rows = tc_token_lane_rows(T, N, K);
     CUtensorMap mw, mx;
     if (rb_tensor_map_bf16(W, N, K, ldw, rows, &mw)) return -1;
     if (rb_tensor_map_bf16(X, T, K, ldx, 128, &mx)) return -1;

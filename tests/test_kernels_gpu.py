@@ -89,6 +89,17 @@ def test_gemm_tiles_of_every_width(T, N, K, rows):
         ops.set_gemm_tile_features(old)
 
 
+def test_gemm_tile_width_of_shallow_products():
+    """Up to three k-steps a product whose tiles of 256 rows leave half of the SMs idle runs in tiles of 64; deeper ones by their
+    rounds."""
+    from reinfer_b200 import ops
+    for T, N in ((400, 2560), (1024, 1536), (300, 4096), (1300, 1024), (257, 64)):
+        for K in (8, 64, 128, 192):
+            assert ops.lib().rb_gemm_token_lane_rows(T, N, K) == 64
+    for T, N, K, rows in ((400, 2560, 512, 144), (1024, 1536, 256, 144), (2048, 4096, 64, 256), (2048, 2560, 9728, 144), (2048, 4096, 4096, 256)):
+        assert ops.lib().rb_gemm_token_lane_rows(T, N, K) == rows, (T, N, K)
+
+
 def _many_token_tiles(ops, T, N, K):
     a = rnd(T, K, dtype=torch.bfloat16, seed=1)
     w = rnd(N, K, dtype=torch.bfloat16, scale=0.05, seed=2)
