@@ -539,12 +539,8 @@ static int fa_group_chunk(int G) {                             // largest diviso
 template <int D, bool VK, int BN = FA_BN, int DO = D, int MINB = 1>
 static int fa_launch_prefill_as(const FaArgs& a, int n_tiles, cudaStream_t s) {
     const size_t smem = (size_t)FA_BM * FaSmem<D>::STRIDE + 2 * fa_stage<D, VK, BN>();
-    static bool done = false;
-    if (!done) {
-        cudaError_t e = cudaFuncSetAttribute(fa_prefill_kernel<D, VK, BN, DO, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        done = true;
-    }
+    static RbPerDevice limit;
+    if (int e = rb_allow_shared(limit, fa_prefill_kernel<D, VK, BN, DO, MINB>, smem)) return e;
     return rb_launch(fa_prefill_kernel<D, VK, BN, DO, MINB>, dim3(n_tiles, a.KH * a.chunks), dim3(FA_THREADS), smem, s, a);
 }
 template <int D>
@@ -553,13 +549,7 @@ static int fa_launch_prefill(const FaArgs& a, int n_tiles, cudaStream_t s) {
         // Tiles of 32 keys and 192 columns of sums put three CTAs on a SM (168 registers, 66 KB) where the plain shape puts
         // two: more warps to hide the products' latency behind, twice the barriers a key.  It pays once the grid fills the
         // device several times over (measured: 18 % faster at 7 CTAs a SM, 4 % slower at 3.5).
-        static int sms = 0;
-        if (sms == 0) {
-            int dev = 0;
-            cudaGetDevice(&dev);
-            if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-        }
-        if (a.v_in_k && a.dv <= 192 && (long long)n_tiles * a.KH * a.chunks >= 6LL * sms)
+        if (a.v_in_k && a.dv <= 192 && (long long)n_tiles * a.KH * a.chunks >= 6LL * rb_sm_count())
             return fa_launch_prefill_as<256, true, 32, 192, 3>(a, n_tiles, s);
     }
     return a.v_in_k ? fa_launch_prefill_as<D, true>(a, n_tiles, s) : fa_launch_prefill_as<D, false>(a, n_tiles, s);
@@ -569,12 +559,8 @@ static int fa_launch_decode_as(const FaArgs& a, cudaStream_t s) {
     const size_t pipe = (size_t)NST * fa_stage<D, VK>();
     const size_t merge = ((size_t)FA_WARPS * 16 * (D + 3) + 16) * sizeof(float);    // parts, maxima, sums, factors, 1 / sum
     const size_t smem = 16 * FaSmem<D>::STRIDE + (pipe > merge ? pipe : merge);
-    static bool done = false;
-    if (!done) {
-        cudaError_t e = cudaFuncSetAttribute(fa_decode_kernel<D, NST, VK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        done = true;
-    }
+    static RbPerDevice limit;
+    if (int e = rb_allow_shared(limit, fa_decode_kernel<D, NST, VK>, smem)) return e;
     return rb_launch(fa_decode_kernel<D, NST, VK>, dim3(a.n_entries, a.KH * a.chunks, a.n_splits), dim3(FA_THREADS), smem, s, a);
 }
 // (a key tile alone leaves room for one more stage)

@@ -689,12 +689,8 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
 
 template <int OPTIONS>
 static int fc_launch(dim3 grid, size_t smem, cudaStream_t s, const CUtensorMap& map, const FcArgs& a) {
-    static bool done = false;                          // once: the call costs the host some microseconds, as much as a launch
-    if (!done) {
-        const cudaError_t e = cudaFuncSetAttribute(fa_prefill_tc_kernel<OPTIONS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
-        done = true;
-    }
+    static RbPerDevice limit;
+    if (int e = rb_allow_shared(limit, fa_prefill_tc_kernel<OPTIONS>, smem)) return e;
     return rb_launch(fa_prefill_tc_kernel<OPTIONS>, grid, dim3(FC_THREADS), smem, s, map, a);
 }
 

@@ -833,15 +833,11 @@ static int ft_launch(const CUtensorMap& map, const FtArgs& a, cudaStream_t s) {
     static_assert(sizeof(FtShared) <= 256, "the cluster's receive buffers start 256 bytes behind the barriers");
     // stages, Q, barriers, and what the other splits of a cluster send: [split][Gc][dq] results + [split][16] log-sum-exps
     constexpr size_t smem = ft_decode_smem<HALVES, NST, KONLY>();
-    static bool done = false;
-    if (!done) {
-        cudaError_t e = cudaFuncSetAttribute(fa_decode_tma_kernel<HALVES, NST, P5, KONLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        // clusters of more than 8 CTAs (up to 16 splits merge themselves) are not portable: the kernel has to allow them
-        e = cudaFuncSetAttribute(fa_decode_tma_kernel<HALVES, NST, P5, KONLY>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (e != cudaSuccess) return (int)e;
-        done = true;
-    }
+    static RbPerDevice limit;
+    // clusters of more than 8 CTAs (up to 16 splits merge themselves) are not portable: the kernel has to allow them
+    if (int e = rb_allow_shared(limit, fa_decode_tma_kernel<HALVES, NST, P5, KONLY>, smem, [] {
+            return cudaFuncSetAttribute(fa_decode_tma_kernel<HALVES, NST, P5, KONLY>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        })) return e;
     const dim3 grid(a.KH * a.chunks, a.n_entries, a.n_splits);
     if (a.cluster_merge)
         return rb_launch_cluster(fa_decode_tma_kernel<HALVES, NST, P5, KONLY>, grid, dim3(FT_THREADS), dim3(1, 1, a.n_splits), smem, s, map, a);
@@ -914,12 +910,8 @@ extern "C" int rb_fa_decode_tma(const void* q, const void* cache, long long num_
 template <int HALVES, int NST>
 static int ft_launch_prefill(const CUtensorMap& map, const FtArgs& a, int n_tiles, cudaStream_t s) {
     constexpr size_t smem = (size_t)NST * 2 * HALVES * FT_HALF_BYTES + HALVES * 64 * 128 + sizeof(FtShared) + 1024;
-    static bool done = false;
-    if (!done) {
-        cudaError_t e = cudaFuncSetAttribute(fa_prefill_tma_kernel<HALVES, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        done = true;
-    }
+    static RbPerDevice limit;
+    if (int e = rb_allow_shared(limit, fa_prefill_tma_kernel<HALVES, NST>, smem)) return e;
     return rb_launch(fa_prefill_tma_kernel<HALVES, NST>, dim3(n_tiles, a.KH * a.chunks), dim3(FT_THREADS), smem, s, map, a);
 }
 

@@ -10,6 +10,7 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 #include <stdio.h>
+#include "per_device.h"
 
 enum RbDtype { RB_F32 = 0, RB_BF16 = 1 };
 
@@ -114,6 +115,35 @@ static inline int rb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
     if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
     return (int)cudaGetLastError();
+}
+
+// That much dynamic shared memory for a kernel on the present device, and what else `more` sets there (a function that returns a
+// cudaError_t).  Asked for once per kernel and device, whose record is `limit`: the calls cost the host as much as a launch.
+template <typename Kernel, typename More>
+static inline int rb_allow_shared(RbPerDevice& limit, Kernel kernel, size_t bytes, More&& more) {
+    int dev = 0;
+    int e = (int)cudaGetDevice(&dev);
+    if (!e) e = limit.raise(dev, bytes, [&] {
+        const cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        return (int)(r == cudaSuccess ? more() : r);
+    });
+    if (e) (void)cudaGetLastError();
+    return e;
+}
+template <typename Kernel>
+static inline int rb_allow_shared(RbPerDevice& limit, Kernel kernel, size_t bytes) {
+    return rb_allow_shared(limit, kernel, bytes, [] { return cudaSuccess; });
+}
+
+// Streaming multiprocessors of the present device (148, a B200's, where there is none to ask).
+static inline int rb_sm_count() {
+    static std::atomic<int> counts[RB_MAX_DEVICES];
+    int dev = -1, n = 0;
+    const bool kept = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < RB_MAX_DEVICES;
+    if (kept && (n = counts[dev].load(std::memory_order_relaxed)) > 0) return n;
+    if (dev < 0 || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) { (void)cudaGetLastError(); return 148; }
+    if (kept) counts[dev].store(n, std::memory_order_relaxed);
+    return n;
 }
 
 // The ordinary way: after everything before it has ended.  For a long kernel of about as many CTAs as there are SMs behind a kernel

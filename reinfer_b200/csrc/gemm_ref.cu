@@ -337,25 +337,13 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
     }
 }
 
-// Both forms of a kernel (store, add) may use that much dynamic shared memory.
-template <typename Kernel>
-static int f32_allow_shared(Kernel store, Kernel add, size_t bytes) {
-    cudaError_t e = cudaFuncSetAttribute(store, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(add, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) (void)cudaGetLastError();
-    return (int)e;
-}
-
 template <int BM, int BN, int TM, int TN, int STAGES>
 static int gemm_f32_tile(const float* A, const float* W, float* C, int accumulate, int M, int N, int K, long long lda,
                          long long ldw, long long ldc, cudaStream_t s) {
     using Tile = F32Tile<BM, BN, TM, TN, STAGES>;
     auto kernel = accumulate ? gemm_f32_tile_kernel<BM, BN, TM, TN, STAGES, 1> : gemm_f32_tile_kernel<BM, BN, TM, TN, STAGES, 0>;
-    static bool done = false;                                       // once: the calls cost the host as much as a launch
-    if (!done) {
-        if (int e = f32_allow_shared(gemm_f32_tile_kernel<BM, BN, TM, TN, STAGES, 0>, gemm_f32_tile_kernel<BM, BN, TM, TN, STAGES, 1>, Tile::SMEM)) return e;
-        done = true;
-    }
+    static RbPerDevice limits[2];                                   // of the form that stores and the one that adds
+    if (int e = rb_allow_shared(limits[accumulate ? 1 : 0], kernel, Tile::SMEM)) return e;
     return rb_launch(kernel, dim3(rb_ceil_div(M, BM), rb_ceil_div(N, BN)), dim3(Tile::THREADS), Tile::SMEM, s, A, W, C, M, N, K, lda, ldw, ldc);
 }
 
@@ -363,11 +351,8 @@ template <int TM>
 static int gemm_f32_few(const float* A, const float* W, float* C, int accumulate, int M, int N, int K, long long lda,
                         long long ldw, long long ldc, cudaStream_t s) {
     auto kernel = accumulate ? gemm_f32_few_kernel<TM, 1> : gemm_f32_few_kernel<TM, 0>;
-    static bool done = false;                                       // once: the calls cost the host as much as a launch
-    if (!done) {
-        if (int e = f32_allow_shared(gemm_f32_few_kernel<TM, 0>, gemm_f32_few_kernel<TM, 1>, F32Few<TM>::SMEM)) return e;
-        done = true;
-    }
+    static RbPerDevice limits[2];                                   // of the form that stores and the one that adds
+    if (int e = rb_allow_shared(limits[accumulate ? 1 : 0], kernel, F32Few<TM>::SMEM)) return e;
     return rb_launch(kernel, dim3(rb_ceil_div(M, 2 * TM), rb_ceil_div(N, 16)), dim3(F32_SEGMENTS * 32), F32Few<TM>::SMEM, s, A, W, C, M, N, K, lda, ldw, ldc);
 }
 
@@ -473,11 +458,8 @@ static int gemm_f32_wide(const float* A, const float* W, float* C, int accumulat
                          long long ldw, long long ldc, cudaStream_t s) {
     constexpr size_t smem = (2 * 2 * 16 * F32W_ROW + 64 * 256) * sizeof(float);
     auto kernel = accumulate ? gemm_f32_wide_kernel<1> : gemm_f32_wide_kernel<0>;
-    static bool done = false;                                       // once: the calls cost the host as much as a launch
-    if (!done) {
-        if (int e = f32_allow_shared(gemm_f32_wide_kernel<0>, gemm_f32_wide_kernel<1>, smem)) return e;
-        done = true;
-    }
+    static RbPerDevice limits[2];                                   // of the form that stores and the one that adds
+    if (int e = rb_allow_shared(limits[accumulate ? 1 : 0], kernel, smem)) return e;
     // (begun early, its CTAs would go where the kernel before leaves room, two to an SM beside idle ones)
     return rb_launch_after(kernel, dim3(rb_ceil_div(M, 128), rb_ceil_div(N, 128)), dim3(256), smem, s, A, W, C, M, N, K, lda, ldw, ldc);
 }

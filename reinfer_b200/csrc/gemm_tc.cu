@@ -1077,16 +1077,9 @@ static int launch_tc_persistent(const CUtensorMap& mw, const CUtensorMap& mx, vo
                                 int mode, cudaStream_t s, const TcHeads& hd, const TcRows& rs) {
     constexpr size_t smem = (size_t)STAGES * ((MODE ? ROWS : TC_BM) * TC_BK * 2 + BN * TC_BK * 2) + sizeof(TcPersistShared) + 1024;
     static_assert(smem <= 232448, "stages beyond the shared memory of an SM");
-    static bool configured = false;
-    static int sms = 0;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_persistent_kernel<BN, STAGES, MODE, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        configured = true;
-    }
+    static RbPerDevice limit;
+    if (int e = rb_allow_shared(limit, gemm_tc_persistent_kernel<BN, STAGES, MODE, ROWS>, smem)) return e;
+    const int sms = rb_sm_count();
     const int t_tiles = rb_ceil_div(T, BN), n_tiles = rb_ceil_div(N, (MODE == 2 || MODE == 3) ? ROWS : MODE == 1 ? ROWS / 2 : TC_BM);
     const int total = t_tiles * n_tiles;
     const int grid = total < sms ? total : sms;
@@ -1255,13 +1248,11 @@ static int launch_tc_gated_stream(const void* X, const void* Wgu, void* act, int
     constexpr size_t smem = (size_t)STAGES * (2 * TCS_ROWS * TC_BK * 2 + XROWS * TC_BK * 2) + (128 - XROWS) * TC_BK * 2 +
                             sizeof(TcStreamShared) + 1024;
     static_assert(smem <= 113 * 1024, "two CTAs to an SM");
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_gated_stream_kernel<STAGES, XROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        (void)cudaFuncSetAttribute(gemm_tc_gated_stream_kernel<STAGES, XROWS>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        configured = true;
-    }
+    static RbPerDevice limit;
+    if (int e = rb_allow_shared(limit, gemm_tc_gated_stream_kernel<STAGES, XROWS>, smem, [] {
+            (void)cudaFuncSetAttribute(gemm_tc_gated_stream_kernel<STAGES, XROWS>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+            return cudaSuccess;
+        })) return e;
     CUtensorMap mw, mx;
     if (rb_tensor_map_bf16(Wgu, (long long)ex.glu.up_row + F, K, ldw, TCS_ROWS, &mw)) return -1;
     if (rb_tensor_map_bf16(X, T, K, ldx, XROWS, &mx)) return -1;
@@ -1369,14 +1360,12 @@ static int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, void* C, floa
                      long long ldc, int mode, int want_splits, const TcExtra& ex, cudaStream_t s,
                      bool keep_partials = false) {
     constexpr size_t smem = (size_t)STAGES * ((DUAL ? 2 : 1) * TC_BM * TC_BK * 2 + BN * TC_BK * 2) + sizeof(TcShared) + 1024;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, STAGES, DUAL, MORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        // the whole of the SM's memory as shared memory, so that two CTAs of the small-tile kernels fit beside each other
-        (void)cudaFuncSetAttribute(gemm_tc_kernel<BN, STAGES, DUAL, MORE>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        configured = true;
-    }
+    static RbPerDevice limit;
+    // the whole of the SM's memory as shared memory, so that two CTAs of the small-tile kernels fit beside each other
+    if (int e = rb_allow_shared(limit, gemm_tc_kernel<BN, STAGES, DUAL, MORE>, smem, [] {
+            (void)cudaFuncSetAttribute(gemm_tc_kernel<BN, STAGES, DUAL, MORE>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+            return cudaSuccess;
+        })) return e;
     const int total_kb = rb_ceil_div(K, TC_BK);
     const int t_tiles = rb_ceil_div(T, BN), n_tiles = rb_ceil_div(N, TC_BM);
     const int tiles = t_tiles * n_tiles;

@@ -358,12 +358,9 @@ static int recurrence_launch(const RecurArgs& A, int n_entries, cudaStream_t st)
     a.tile = (R::FLOATS + COLS) * 16 * sizeof(float) * (AHEAD ? 2 : 1) > 160 * 1024 || RP >= 64 ? 8 : 16;
     const size_t smem = (size_t)a.tile * ((R::FLOATS + COLS) * (AHEAD ? 2 : 1) + COLS * SPLIT) * sizeof(float);
     dim3 grid(rb_ceil_div(a.dv, COLS), a.H, n_entries);
-    static bool done = false;                          // two buffers may pass the default limit of dynamic shared memory
-    if (!done && smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(recurrence_kernel<TA, FORM, SPLIT, RP, AHEAD, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        done = true;
-    }
+    static RbPerDevice limit;                          // two buffers may pass the default limit of dynamic shared memory
+    if (smem > 48 * 1024)
+        if (int e = rb_allow_shared(limit, recurrence_kernel<TA, FORM, SPLIT, RP, AHEAD, COLS>, smem)) return e;
     if (AHEAD) {
         a.rec_floats = R::FLOATS + rb_ceil_div(a.dv, RR_COLS) * RR_COLS;
         const long long warps = (long long)a.n_tokens * a.H;

@@ -184,12 +184,9 @@ template <typename TX, typename TO>
 static int lp_launch(size_t smem, int T, cudaStream_t s, const TX* x, long long x_stride, int na, int nc, int nr, const float* wa,
                      const float* wc, float eps, const int* positions, const float* freq, int rot, float mag, int layout, const int* kv_slot,
                      TO* a_out, TO* cache, int page_size) {
-    static size_t allowed = 48 * 1024;
-    if (smem > allowed) {
-        cudaError_t e = cudaFuncSetAttribute(latent_prep_kernel<TX, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        allowed = smem;
-    }
+    static RbPerDevice limit;
+    if (smem > 48 * 1024)
+        if (int e = rb_allow_shared(limit, latent_prep_kernel<TX, TO>, smem)) return e;
     return rb_launch(latent_prep_kernel<TX, TO>, dim3(T), dim3(LP_THREADS), smem, s, x, x_stride, na, nc, nr, wa, wc, eps,
                      positions, freq, rot, mag, layout, kv_slot, a_out, cache, page_size);
 }

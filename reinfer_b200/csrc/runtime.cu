@@ -134,7 +134,6 @@ extern "C" int rb_attn_error(int);
 extern "C" int rb_attn_tc_error(int);
 extern "C" int rb_selftest_error(int);
 
-#define RB_MAX_DEVICES 64
 static int* g_status_host[RB_MAX_DEVICES] = {nullptr};
 static std::mutex g_status_mu;
 

@@ -282,3 +282,54 @@ def test_prenorm_block_hands_sums_and_prepared_rows_on():
     out = block.forward(ctx, x, None, None)
     assert [e[2] for e in log if e[0] == "mixer"] == [None]          # the mixer was told of no norm
     assert isinstance(out, PreparedRows)                            # the ffn still prepares for the next block's norm
+
+
+def test_kernel_limits_are_granted_once_per_device(tmp_path):
+    """The record behind every kernel's shared-memory limit: a device's first call asks for it, whatever was granted on another
+    device, a larger one asks again, a failed one does not count, and threads that come at once ask once."""
+    import ctypes
+    import os
+    import subprocess
+    import threading
+    from reinfer_b200.csrc import build
+    src, out = tmp_path / "limits.cpp", tmp_path / "limits.so"
+    src.write_text('#include "per_device.h"\nstatic RbPerDevice limit;\n'
+                   'extern "C" int raise_limit(int dev, long want, int (*set)()) { return limit.raise(dev, (size_t)want, set); }\n')
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-pthread", "-I", os.path.dirname(build.__file__), str(src), "-o", str(out)], check=True)
+    raise_limit = ctypes.CDLL(str(out)).raise_limit
+    callback = ctypes.CFUNCTYPE(ctypes.c_int)
+    calls, answer = [], [0]
+
+    def count():
+        calls.append(1)
+        return answer[0]
+
+    def asked(dev, want):
+        before, rc = len(calls), raise_limit(dev, ctypes.c_long(want), fn)
+        return rc, len(calls) - before
+
+    fn = callback(count)
+    assert asked(0, 100) == (0, 1) and asked(0, 100) == (0, 0) and asked(0, 60) == (0, 0)
+    assert asked(1, 100) == (0, 1) and asked(63, 60) == (0, 1)         # another device has been granted nothing yet
+    assert asked(0, 101) == (0, 1) and asked(0, 100) == (0, 0)
+    assert asked(64, 100) == (0, 1) and asked(64, 100) == (0, 1) and asked(-1, 1) == (0, 1)      # beyond the table: asked every time
+    answer[0] = 7
+    assert asked(2, 100) == (7, 1) and asked(2, 100) == (7, 1)
+    answer[0] = 0
+    assert asked(2, 100) == (0, 1) and asked(2, 100) == (0, 0)
+    before = len(calls)
+    threads = [threading.Thread(target=raise_limit, args=(5, ctypes.c_long(9), fn)) for _ in range(16)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert len(calls) == before + 1
+
+
+def test_no_kernel_limit_is_remembered_for_the_whole_process():
+    """Every cudaFuncSetAttribute of the kernels stands behind a record per device, or runs at every call."""
+    import os
+    import re
+    from reinfer_b200.csrc import build
+    for name in build.sources():
+        with open(os.path.join(os.path.dirname(build.__file__), name)) as f:
+            text = f.read()
+        assert not re.search(r"static (bool|size_t|int) \w+ = [^;]*;[^}]{0,200}cudaFuncSetAttribute", text), name
