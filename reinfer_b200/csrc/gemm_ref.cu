@@ -473,7 +473,8 @@ static int gemm_f32_dispatch(const float* A, const float* W, float* C, int accum
     if (M <= 2) return gemm_f32_few<1>(A, W, C, accumulate, M, N, K, lda, ldw, ldc, s);
     if (M <= 4) return gemm_f32_few<2>(A, W, C, accumulate, M, N, K, lda, ldw, ldc, s);
     if (M <= 16) return gemm_f32_few<4>(A, W, C, accumulate, M, N, K, lda, ldw, ldc, s);
-    auto busiest = [&](int bm, int bn) { return (long long)rb_ceil_div((long long)rb_ceil_div(M, bm) * rb_ceil_div(N, bn), 148); };
+    const int sms = rb_sm_count();
+    auto busiest = [&](int bm, int bn) { return (long long)rb_ceil_div((long long)rb_ceil_div(M, bm) * rb_ceil_div(N, bn), sms); };
     const long long wide = busiest(128, 128) == 1 ? 140 : 134 * busiest(128, 128);
     const long long tile = 80 * busiest(64, 128);
     const long long mid = busiest(32, 64) == 1 ? 35 : 26 * busiest(32, 64);

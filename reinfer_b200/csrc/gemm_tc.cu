@@ -1289,9 +1289,7 @@ static int tc_capacity(int sp, size_t smem) {
     static int cache[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     if (cache[sp]) return cache[sp];
     constexpr int MINB = BN <= 64 ? 2 : 1;                          // the kernel's __launch_bounds__
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = rb_sm_count();
     (void)cudaFuncSetAttribute(tc_occupancy_twin<MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int n = 0;
     if (sp == 1) {
@@ -1471,9 +1469,7 @@ static TcRows tc_rows(const TcExtra& ex) {
 #define TC_SHALLOW (3 * TC_BK)
 static int tc_token_lane_rows(int T, int N, int K) {
     if (g_tc_tile_feats) return g_tc_tile_feats;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = rb_sm_count();
     const long long t_tiles = rb_ceil_div(T, 128);
     if (K <= TC_SHALLOW && 2 * rb_ceil_div(N, 256) * t_tiles <= sms) return 64;
     int best = 256;
@@ -1556,9 +1552,7 @@ extern "C" int rb_gemm_bf16(const void* X, const void* W, void* C, int c_dtype, 
         const bool flip = g_tc_token_lanes != 0;
         if (flip) return launch_tc_token_lanes(X, W, C, T, N, K, ldx, ldw, ldc, mode, tc_rows(ex), s);
         if (row_sumsq) RB_REFUSE("gemm: row factors over %d tokens need the token-lane persistent product", T);
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const int sms = rb_sm_count();
         const long long n_tiles = rb_ceil_div(N, TC_BM);
         const double c256 = (double)rb_ceil_div((long long)rb_ceil_div(T, 256) * n_tiles, sms) * 256.0;
         const double c128 = (double)rb_ceil_div((long long)rb_ceil_div(T, 128) * n_tiles, sms) * 128.0 * 1.36;
@@ -1719,9 +1713,7 @@ extern "C" int rb_gemm_qkv_heads_stream(const void* X, const void* W, int T, int
 // 64-wide blocks of K each.  No cluster is involved, so nothing limits the count but the work.
 extern "C" int rb_gemm_partials_plan(int T, int N, int K) {
     if (T <= 0 || N <= 0 || K <= 0) return 1;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = rb_sm_count();
     const int bn = tc_bn(T);
     // four fifths of the slots: the kernels after this one then find room to start early and fetch their own
     // first tiles while this one drains (measured inside whole decode steps; REINFER_B200_PARTIAL_FILL for tuning)
