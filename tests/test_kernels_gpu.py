@@ -817,6 +817,43 @@ def test_prompt_attention_over_pages_of_every_size(page, window):
     assert ops.kernel_error() == 0
 
 
+@pytest.mark.parametrize("page", [8, 64])
+@pytest.mark.parametrize("options", ["cap", "penalty", "bias", "sink", "gate", "gate_heads", "chunk", "cap penalty", "cap bias window", "penalty bias sink",
+                                     "penalty chunk", "cap penalty bias sink gate"])
+def test_prompt_attention_options_against_64_bits(options, page):
+    """Each option of the tcgen05 attention alone and several together (one instantiation an option, and a general one), with keys that
+    end in the first half of a 128-key tile, in the second and on its edge.  P and the result are rounded to bfloat16: three half units
+    of 2^-8 of the largest value; a number of the table of biases is reached by its last column too."""
+    from reinfer_b200 import ops
+    QH, KH, lens, q_lens = 8, 2, [833, 193, 129, 128, 64], [420, 193, 70, 128, 33]
+    q, cache, bt, kv = prompt_attention_setup(lens, q_lens, QH, KH, page, 31)
+    r = lambda *shape, seed: rnd(*shape, seed=seed)
+    kw = {}
+    if "cap" in options:
+        kw["softcap"] = 3.0
+    if "penalty" in options:
+        kw["penalty"] = (r(QH, seed=1).abs(), r(QH, seed=2).abs())
+    if "bias" in options:
+        kw["bias"] = 0.5 * r(QH, 90, seed=3)
+    if "sink" in options:
+        kw["sink"] = r(QH, seed=4) + 3.0
+    if "gate" in options.split():
+        kw["gate"] = r(sum(q_lens), QH * 128, seed=5)
+    if "gate_heads" in options:
+        kw["gate"] = r(sum(q_lens), QH, seed=6)
+    window, chunk = 300 * ("window" in options), 192 * ("chunk" in options)
+    as_int = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    out, scale = torch.full_like(q, math.nan), 128 ** -0.5
+    more = ops.AttentionExtras(softcap=kw.get("softcap", 0.0), sink=kw.get("sink"), gate=kw.get("gate"), gate_heads="gate_heads" in options)
+    ops.fa_prefill_tc(q, cache, bt.to(DEV), as_int([sum(q_lens[:r]) for r in range(len(lens) + 1)]), as_int(lens), out, 0, len(lens), q_lens,
+                      QH, KH, 128, page, window, scale, chunk=chunk, penalty=kw.get("penalty"), bias=kw.get("bias"), more=more)
+    if "gate_heads" in options:
+        kw["gate"] = kw["gate"].repeat_interleave(128, dim=1)
+    ref = prompt_attention_truth(q, kv, q_lens, scale, window=window, chunk=chunk, **kw)
+    assert (out.double() - ref).abs().max().item() <= 3 * 2.0 ** -9 * max(x[:, 1].float().abs().max().item() for x in kv)
+    assert ops.kernel_error() == 0
+
+
 def test_attention_finds_one_far_key():
     """One key among hundreds gets a score that stands out; the output must be its value."""
     from reinfer_b200 import ops
