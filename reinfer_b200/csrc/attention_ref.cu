@@ -1,11 +1,12 @@
 // The plain attention over the paged cache: any number of new tokens per request,
-// causal, grouped heads, optional window.  One warp per (token, query head) walks the
-// keys of its request in ascending order, in blocks of 32 that are aligned to absolute
-// positions, with one online-softmax update per block.  The sequence of operations for
-// a token depends only on its position (and the window), never on how the request was
-// cut into steps, on the batch, or on the page size - so this kernel gives the same
-// bits under every cut.  It is the attention of the 32-bit path and the yardstick of
-// the faster bfloat16 kernels.
+// causal, grouped heads, optional window.  Keys are walked in blocks of 32 that are aligned
+// to absolute positions, with one online-softmax update per block: by several warps of a
+// CTA per (token, query heads of a kv head), their results added in a fixed order, where
+// rows are multiples of four numbers (the second kernel below), else in ascending order by
+// one warp per (token, query head).  The sequence of operations for a token depends only
+// on its position and its mask, never on how the request was cut into steps, on the
+// batch, or on the page size - so the same bits come out under every cut.  It is the
+// attention of the 32-bit path and the yardstick of the faster bfloat16 kernels.
 // Beyond the plain form it takes: a value head size of its own (dv != d), a chunk mask (a token sees the
 // keys of its own chunk of `chunk` positions, counted from position 0), a logarithmic distance penalty per
 // query head (score -= r1[h] * ln(1 + r2[h] * (i - j))), a learned bias by distance (score += bias[h][min(i - j,
@@ -126,9 +127,9 @@ paged_attention_ref_kernel(const TA* __restrict__ q, const TC* __restrict__ cach
     }
 }
 
-// The same attention with the keys of a (token, query heads of one kv head) shared out among the 8 warps of a CTA, for head
-// sizes that are multiples of four: warp w walks the 32-key blocks whose index is w modulo 8, in ascending order, with its own
-// running maximum; the eight partial results are added in warp order.  Blocks are aligned to absolute positions, so what is
+// The same attention with the keys of a (token, query heads of one kv head) shared out among the WARPS warps of a CTA (8; fewer for
+// short masks), for head sizes that are multiples of four: warp w walks the 32-key blocks whose index is w modulo WARPS, in
+// ascending order, with its own running maximum; the partial results are added in warp order.  Blocks are aligned to absolute positions, so what is
 // added in which order still depends on nothing but the token's position and mask.  A lane scores one key for G query heads
 // at once (rows read 16 bytes at a time, the queries broadcast from shared memory), and sums four columns of the values.
 // Bound by latency: a block's 32 scores are one chain of d loads and FMAs per lane.  727 tokens in four prompts of 40 to 300, 32

@@ -27,11 +27,13 @@
 // room for a third tile of keys, so what waits for what decides: keys have slots of their own, refilled as soon as the scores
 // that read them are there, a tile ahead of their use; values are refilled behind their product and needed half a tile later.
 //
-// What bounds a key tile now: the special-function units.  A tile's 2 x 128 x 128 exponentials take them 2,048 cycles of the
-// about 3,900 that a tile takes; its products take the tensor cores 2,048.  (-DRB_TIMELINE: lane 0 of every warp adds up its
-// waits and its work; a row warp spends 2,530 in the exponentials' passes, 220 waiting for scores, 230 for its P buffer.)
+// What bounds a key tile now: a row warp's own work.  Of the about 3,900 cycles that a tile takes it is at work 3,750: 2,530 in the
+// exponentials' passes, about 1,200 outside of them (scores into registers, edge tests, fences and arrivals); it waits 220 for
+// scores and 230 for its P buffer.  (-DRB_TIMELINE: lane 0 of every warp adds up its waits and its work.)  The special-function
+// units have 2,048 cycles of exponentials a tile and the tensor cores 2,048 of products, about half of the time each.
 // 2,048 tokens behind 14,336 others, 32 query over 8 kv heads: 525 us (980 TFLOP/s); tiles of 64 keys with two score buffers
-// took 663 (a product of 128 x 64 costs nearly what one of 128 x 128 does), 128 keys in one ring of keys and values 642.
+// took 663, 128 keys in one ring of keys and values 642 (128 keys alone 1 % more than 663: what that gave was the options' code out
+// of the loop and one copy of the exponentials').
 // Scaling, sums and maxima are packed or three-input instructions, and the code of the options is in instantiations of its
 // own, for the rows' loop has to fit the instruction cache: with all options in it, a fifth of the rows' stalls were
 // instruction fetches.  Built, measured, left out: two threads per row (the row's maximum agreed through shared memory: 11 %
@@ -53,7 +55,7 @@
 #define FC_ROWS 128                           // query rows per row tile
 #define FC_TILES 2                            // row tiles per CTA
 #define FC_D 128
-#define FC_THREADS 384                        // a control group (TMA warp, MMA warp, two idle) and two groups of four row warps
+#define FC_THREADS 384                        // a control group (TMA, scores of tile A, weighted sums, scores of tile B) and two groups of four row warps
 #define FC_SLOTS 6                            // half tiles: keys of even tiles in slots 0, 1, of odd tiles in 2, 3; values in 4, 5
 #define FC_KSLOT(tile) (((tile) & 1) * 2)
 #define FC_VSLOT(half) (4 + ((half) & 1))
@@ -144,8 +146,9 @@ __device__ __forceinline__ void fc_commit_lead(uint32_t bar, uint32_t lead) {
 
 // 2^x by the special-function unit alone: one instruction (exp2f adds range handling around it, and so does
 // ex2.approx without .ftz: a compare and two multiplications per call for results below 2^-126, which are flushed to
-// zero here - P is rounded to bfloat16 anyway).  The arguments are <= 0 or -inf, where it is accurate to two units in
-// the last place.
+// zero here - P is rounded to bfloat16 anyway).  Accurate to two units in the last place.  The arguments that count are at most
+// FC_RESCALE, or -inf; a pass against an old maximum may see any larger one and overflow: such a maximum moves, and the pass
+// is done again.
 __device__ __forceinline__ float fc_ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -229,7 +232,7 @@ extern "C" int rb_fa_tc_trace(unsigned long long* buf) { return (int)cudaMemcpyT
 
 // OPTIONS: which options on the scores there may be (FC_CAP | FC_PENALTY | FC_BIAS).  They are instantiations because their
 // unrolled code would stand in the rows' loop: with all of it there the loop did not fit the instruction cache and the rows
-// spent two fifths of a key tile fetching code that they jumped over.
+// spent a fifth of a key tile fetching code that they jumped over.
 #define FC_CAP 1
 #define FC_PENALTY 2
 #define FC_BIAS 4

@@ -228,8 +228,9 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
 // Few tokens (2 * TM per CTA): 16 features per CTA, warp w sums segment w.  A warp has a pipeline of its own - it copies its rows'
 // next 32 k itself and waits for nobody - and is 16 feature lanes x 2 halves of the tokens; a weight that has arrived is read
 // twice from shared memory.  The sums of the segments meet in shared memory.
-// Bound by the stream of weights.  4 tokens over 151,936 x 2,560: 272 us (5.7 TB/s; the kernel at the top of this file 2.23 ms);
-// over 19,456 x 2,560: 55 us (430); over 2,560 x 9,728: 39 us (1,056), where 160 CTAs are too few to keep memory busy.
+// Bound by the stream of weights up to four tokens, then by its own loads and FMAs.  Launches back to back, 4 tokens over 151,936 x
+// 2,560: 255 us (6.1 TB/s; the kernel at the top of this file 2.22 ms), 8 tokens 310 to 370; 4 tokens over 19,456 x 2,560: 39 us
+// (424); over 2,560 x 9,728: 34 us (972), where 160 CTAs are too few to keep memory busy.
 #define F32_ROW (F32_UNIT + 4)
 template <int TM>
 struct F32Few {

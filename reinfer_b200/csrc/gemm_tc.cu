@@ -646,7 +646,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
                           void* __restrict__ C, int T, int N, int K, long long ldc, int out_mode, int t_tiles, int n_tiles,
                           TcHeads hd, TcRows rs) {
     // MODE 0: a tile is 128 features (the M operand) x BN tokens.  MODE 1 (the gated pair) and MODE 2: a tile is 128
-    // tokens (the M operand) x ROWS weight rows (the N operand; a multiple of 32 up to 256): ROWS / 2 gate rows and the
+    // tokens (the M operand) x ROWS weight rows (the N operand; a multiple of 16, of 32 for the pair, up to 256): ROWS / 2 gate rows and the
     // ROWS / 2 up rows of the same features, or ROWS features.  A lane of the accumulator is then a token, and the
     // epilogue writes 16 features of it at a time.  Fewer rows leave room for a stage more.
     constexpr bool DUAL = MODE == 1, FLIP = MODE != 0, HEADS = MODE == 3;
@@ -958,7 +958,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
                     }
                 }
             } else if (FLIP) {
-                // a lane is a token; its 256 columns are 256 features
+                // a lane is a token; its columns are the tile's features
                 const int tok = t0 + q * 32 + lane;
                 const bool vec4 = (ldc % 4 == 0) && (((uintptr_t)C & 15) == 0);
 #pragma unroll 1

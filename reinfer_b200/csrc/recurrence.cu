@@ -244,9 +244,10 @@ recurrence_kernel(const RecurArgs A) {
         // compiler may not do that by itself: the stores of the read-out's parts stand between).
         RecurVectors<FORM, RP> x;
         if (RP <= 8 && AHEAD) x.load(recs + r * RPP, VEC, recs + R::NARR * VEC, vs[cl]);
-        // (unrolled, so that handing the fetched vectors on costs no moves; with the copies of a record addressed by warp instead of
-        // by a division per 16 bytes: 895 of 2,048 tokens in three requests, 16 heads, form 1 with 64 x 64 states 279 -> 228 us, form 2
-        // with 128 x 128 460 -> 418, form 0 with 64 x 128 179 -> 162)
+        // (Unrolled, so that handing the fetched vectors on costs no moves; with the copies of a record addressed by warp instead of
+        // by a division per 16 bytes.  A step of 2,048 tokens in portions of 895, 589 and 564, 16 heads: form 1 with 64 x 64 states
+        // 279 -> 228 us, form 2 with 128 x 128 460 -> 418, form 0 with 64 x 128 179 -> 162.  Eight of the twelve instances spill 4 to
+        // 12 bytes for it.)
         constexpr int UNROLL = RP <= 8 && AHEAD ? 4 : 1;
 #pragma unroll UNROLL
         for (int tt = 0; tt < nt; ++tt) {
