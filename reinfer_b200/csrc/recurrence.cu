@@ -7,11 +7,10 @@
 //   form 3 (read before write):    o = (S + diag(u) k v^T)^T q;  S <- diag(g) S + k v^T      (u [H, dk]: the present token's bonus)
 //
 // A column of S (one value channel) evolves on its own, so the work is split by columns: a CTA owns
-// RR_COLS columns of one (request, head), a column is shared by SPLIT adjacent lanes that hold RP rows
-// each in registers, and the two dot products per token are completed by log2(SPLIT) shuffles in a fixed order.
-// SPLIT is 4 where the state's traffic decides (a decode step: a warp then reads whole 32-byte pieces of a state
-// row) and in 32-bit (one summation order, hence the same bits under every cut); long bfloat16 portions take 8 or 16
-// lanes a column - a token's step is a chain of dependent instructions, and more warps with fewer rows each hide it.
+// RR_COLS columns of one (request, head), a column is shared by SPLIT = 4 adjacent lanes that hold RP rows
+// each in registers (a warp then reads whole 32-byte pieces of a state row), and the two dot products per token are
+// completed by two shuffles in a fixed order: one summation order, hence in 32-bit the same bits under every cut.
+// Long bfloat16 portions with more than 32 key channels go four tokens at a time (recurrence_chunk.cu).
 // The CTA walks its request's tokens of this step in order; per tile of tokens all threads first prepare
 // the token vectors in shared memory - the gate from its pre-activation, unit vectors, scales - in float:
 // (a gate is held as g - 1 = expm1(ln g) and applied as S + (g - 1) S, so that a gate near 1 keeps its digits)
@@ -25,45 +24,10 @@
 // over the whole step in parallel, and leaves the vectors in a scratch buffer that the walking CTAs copy tile by
 // tile: the transcendental work then stands neither in the sequential path nor is it repeated by the CTAs that
 // share a head.  Both ways run the same preparation code and give the same bits.
-#include "common.cuh"
+#include "recurrence.cuh"
 
-#define RR_COLS 32                       // value columns of a CTA of the narrow form (the wide form takes 16); records pad v to this
+#define RR_COLS 32                       // value columns of a CTA; records pad v to this
 #define RR_PREP_THREADS 128
-
-struct RecurArgs {
-    const void* q; long long ldq;          // [T, Hk * dk]   (activation dtype)
-    const void* k; long long ldk;          // [T, Hk * dk]
-    const void* v; long long ldv;          // [T, H * dv]
-    const float* z; long long ldz;         // [T, H * dk] gate pre-activation without its bias ([T, H] with z_per_head)
-    const float* z_bias;                   // [H * dk] or null ([H] with z_per_head)
-    int z_per_head;                        // one gate per head and token instead of one per key channel
-    const void* a_pre; long long lda;      // form 1: removal rate before the sigmoid [T, H * dk] (activation dtype)
-    const float* a_bias;                   // form 1: [H * dk] or null
-    const void* b_pre; long long ldb;      // form 2: write strength before the sigmoid [T, H]
-    const float* rate;                     // gate 2: [H]
-    const float* bonus;                    // form 3: [H * dk]
-    float gate_param;                      // gate 0: 1 / tau;  gate 1: c
-    float q_scale;                         // q is multiplied by this (after it was made a unit vector, if it is)
-    int unit_qk;                           // q and k are made unit vectors: x / sqrt(sum x^2 + 1e-6)
-    int gate;
-    float* state;                          // [slots, H, dk, dv]
-    float* out;                            // [T, H, dv]
-    const int* cu_q; const int* entry_slot;
-    int H, Hk, dk, dv, tile;
-    float* prep;                           // [T, H, record] vectors prepared ahead (null: the walking kernel prepares them)
-    int n_tokens;
-    int rec_floats;                        // floats of a record made ahead: the vectors, then v of the head padded to RR_COLS columns
-};
-
-__device__ __forceinline__ void rr_cp_async16(void* dst, const void* src) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void rr_cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void rr_cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-__device__ __forceinline__ float softplus_f(float x) { return fmaxf(x, 0.0f) + log1pf(expf(-fabsf(x))); }
-__device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
 
 // A token's record for one head: the vectors q, k, g - 1 (form 1 also u and a*u), each as SPLIT row slices of RP
 // floats padded to RP + 4 (so that the slices of the lanes that share a column lie in different banks), then the
@@ -106,12 +70,7 @@ __device__ __forceinline__ void recur_prepare(const RecurArgs& A, size_t t, int 
             if (A.z_bias) z += A.z_bias[zi];
             // the gate is kept as g - 1 = expm1(ln g): a gate close to 1 (a memory that lasts thousands of
             // tokens) then keeps the digits of 1 - g that rounding g itself to float would drop
-            float lg;
-            if (A.gate == 0) lg = -softplus_f(-z) * A.gate_param;
-            else if (A.gate == 1) lg = -A.gate_param * sigmoid_f(z);
-            else if (A.gate == 2) lg = -rate * softplus_f(z);
-            else lg = -expf(z);
-            g = expm1f(lg);
+            g = expm1f(recur_log_gate(A, z, rate));
             if (FORM == 3) bonus = fmaf(qv * kv, A.bonus[(size_t)h * dk + i], bonus);
             if (FORM == 1) {
                 float ap = to_f32(((const TA*)A.a_pre)[t * A.lda + (size_t)h * dk + i]);
@@ -244,10 +203,7 @@ recurrence_kernel(const RecurArgs A) {
         // compiler may not do that by itself: the stores of the read-out's parts stand between).
         RecurVectors<FORM, RP> x;
         if (RP <= 8 && AHEAD) x.load(recs + r * RPP, VEC, recs + R::NARR * VEC, vs[cl]);
-        // (Unrolled, so that handing the fetched vectors on costs no moves; with the copies of a record addressed by warp instead of
-        // by a division per 16 bytes.  A step of 2,048 tokens in portions of 895, 589 and 564, 16 heads: form 1 with 64 x 64 states
-        // 279 -> 228 us, form 2 with 128 x 128 460 -> 418, form 0 with 64 x 128 179 -> 162.  Eight of the twelve instances spill 4 to
-        // 12 bytes for it.)
+        // (Unrolled, so that handing the fetched vectors on costs no moves.)
         constexpr int UNROLL = RP <= 8 && AHEAD ? 4 : 1;
 #pragma unroll UNROLL
         for (int tt = 0; tt < nt; ++tt) {
@@ -337,24 +293,20 @@ recurrence_kernel(const RecurArgs A) {
     }
 }
 
-// Lanes per column and rows per lane for a key size: (4, 8..64) is the narrow form; the wide form (long bfloat16
-// portions) is (8, 8) up to 64 key channels, (16, 8) up to 128, (16, 16) up to 256.
-static void recurrence_shape(int dk, bool wide, int* split, int* rp) {
-    if (wide && dk > 32) {
-        *split = dk <= 64 ? 8 : 16;
-        *rp = dk <= 128 ? 8 : 16;
-        return;
-    }
+// Rows of a column per lane, for a key size.
+static int recurrence_rows(int dk) {
     const int need = rb_ceil_div(dk, 4);
-    *split = 4;
-    *rp = need <= 8 ? 8 : need <= 16 ? 16 : need <= 32 ? 32 : 64;
+    return need <= 8 ? 8 : need <= 16 ? 16 : need <= 32 ? 32 : 64;
 }
+// Tokens of a portion up to which the walking kernel prepares its vectors itself.
+extern "C" int rb_recurrence_tile(int dk) { return recurrence_rows(dk) >= 64 ? 8 : 16; }
+// Long portions whose tokens are walked in chunks: 16-bit activations, more key channels than the narrow records' slices hold.
+static bool recurrence_chunked(int dtype, int dk) { return dtype == RB_BF16 && dk > 32; }
 
 template <typename TA, int FORM, int SPLIT, int RP, bool AHEAD>
 static int recurrence_launch(const RecurArgs& A, int n_entries, cudaStream_t st) {
     using R = RecurRecord<FORM, SPLIT, RP>;
-    // the wide form: 16 columns a CTA, so that the CTAs of one long portion spread over twice as many SMs
-    constexpr int COLS = SPLIT > 4 ? 16 : RR_COLS;
+    constexpr int COLS = RR_COLS;
     RecurArgs a = A;
     a.tile = (R::FLOATS + COLS) * 16 * sizeof(float) * (AHEAD ? 2 : 1) > 160 * 1024 || RP >= 64 ? 8 : 16;
     const size_t smem = (size_t)a.tile * ((R::FLOATS + COLS) * (AHEAD ? 2 : 1) + COLS * SPLIT) * sizeof(float);
@@ -375,21 +327,15 @@ static int recurrence_launch(const RecurArgs& A, int n_entries, cudaStream_t st)
     return rb_launch(recurrence_kernel<TA, FORM, SPLIT, RP, AHEAD, COLS>, grid, dim3(COLS * SPLIT), smem, st, a);
 }
 
-template <typename TA, int FORM, bool WIDE_OK>
+template <typename TA, int FORM>
 static int recurrence_dispatch(const RecurArgs& A, int n_entries, int max_q_len, cudaStream_t st) {
-    int tile_probe_split, rp;
-    recurrence_shape(A.dk, false, &tile_probe_split, &rp);
-    const bool ahead = A.prep != nullptr && max_q_len > (rp >= 64 ? 8 : 16);
-    int split;
-    recurrence_shape(A.dk, WIDE_OK && ahead, &split, &rp);
-    if (ahead) {
-        if (WIDE_OK && split == 8) return recurrence_launch<TA, FORM, 8, 8, true>(A, n_entries, st);
-        if (WIDE_OK && split == 16 && rp == 8) return recurrence_launch<TA, FORM, 16, 8, true>(A, n_entries, st);
-        if (WIDE_OK && split == 16) return recurrence_launch<TA, FORM, 16, 16, true>(A, n_entries, st);
+    const int rp = recurrence_rows(A.dk);
+    if (A.prep != nullptr && max_q_len > rb_recurrence_tile(A.dk)) {
         if (rp == 8) return recurrence_launch<TA, FORM, 4, 8, true>(A, n_entries, st);
-        if (rp == 16) return recurrence_launch<TA, FORM, 4, 16, true>(A, n_entries, st);
-        if (rp == 32) return recurrence_launch<TA, FORM, 4, 32, true>(A, n_entries, st);
-        return recurrence_launch<TA, FORM, 4, 64, true>(A, n_entries, st);
+        if (sizeof(TA) == 2) RB_REFUSE("recurrence: %d key channels are walked in chunks", A.dk);
+        if (rp == 16) return recurrence_launch<float, FORM, 4, 16, true>(A, n_entries, st);
+        if (rp == 32) return recurrence_launch<float, FORM, 4, 32, true>(A, n_entries, st);
+        return recurrence_launch<float, FORM, 4, 64, true>(A, n_entries, st);
     }
     if (rp == 8) return recurrence_launch<TA, FORM, 4, 8, false>(A, n_entries, st);
     if (rp == 16) return recurrence_launch<TA, FORM, 4, 16, false>(A, n_entries, st);
@@ -397,24 +343,16 @@ static int recurrence_dispatch(const RecurArgs& A, int n_entries, int max_q_len,
     return recurrence_launch<TA, FORM, 4, 64, false>(A, n_entries, st);
 }
 
-// Floats of scratch per (token, head) that the preparation ahead needs (the largest over the forms of the kernel that
-// this key size can take).
-extern "C" int rb_recurrence_record_floats(int form, int dk, int dv) {
-    int best = 0;
-    for (int wide = 0; wide < 2; ++wide) {
-        int split, rp;
-        recurrence_shape(dk, wide != 0, &split, &rp);
-        const int f = (form == 1 ? 5 : 3) * split * (rp + 4) + 4;
-        best = f > best ? f : best;
-    }
-    return best + rb_ceil_div(dv, RR_COLS) * RR_COLS;
+// Floats of scratch that a step whose longest portion exceeds one tile needs for the vectors prepared ahead.
+extern "C" long long rb_recurrence_scratch_floats(int form, int dtype, int dk, int dv, int H, int n_tokens, int n_entries) {
+    if (recurrence_chunked(dtype, dk)) return recurrence_chunks_scratch(form, dk, dv, H, n_tokens, n_entries);
+    const int record = (form == 1 ? 5 : 3) * 4 * (recurrence_rows(dk) + 4) + 4;
+    return (long long)n_tokens * H * (record + rb_ceil_div(dv, RR_COLS) * RR_COLS);
 }
-// Tokens of a portion up to which the walking kernel prepares its vectors itself.
-extern "C" int rb_recurrence_tile(int dk) { return rb_ceil_div(dk, 4) > 32 ? 8 : 16; }
 
 // form: 0 .. 3 as above.  All row strides in elements.  state [slots, H, dk, dv] float; out [T, H, dv] float.
-// prep: scratch of n_tokens * H * rb_recurrence_record_floats() floats, or null; it is used when max_q_len (the
-// step's longest portion) exceeds one tile.
+// prep: scratch of rb_recurrence_scratch_floats() floats, 16-byte aligned, or null; it is used when max_q_len (the step's longest
+// portion) exceeds one tile.
 extern "C" int rb_recurrence(int form, int gate, int dtype,
                              const void* q, long long ldq, const void* k, long long ldk, const void* v, long long ldv,
                              const float* z, long long ldz, const float* z_bias, int z_per_head,
@@ -439,13 +377,14 @@ extern "C" int rb_recurrence(int form, int gate, int dtype,
     A.state = state; A.out = out; A.cu_q = cu_q; A.entry_slot = entry_slot;
     A.H = H; A.Hk = Hk; A.dk = dk; A.dv = dv; A.tile = 16; A.prep = prep; A.n_tokens = n_tokens; A.rec_floats = 0;
     cudaStream_t st = (cudaStream_t)stream;
-#define RB_RECUR(TA, WIDE) \
-    do { if (form == 0) return recurrence_dispatch<TA, 0, WIDE>(A, n_entries, max_q_len, st); \
-         if (form == 1) return recurrence_dispatch<TA, 1, WIDE>(A, n_entries, max_q_len, st); \
-         if (form == 3) return recurrence_dispatch<TA, 3, WIDE>(A, n_entries, max_q_len, st); \
-         return recurrence_dispatch<TA, 2, WIDE>(A, n_entries, max_q_len, st); } while (0)
-    if (dtype == RB_F32) RB_RECUR(float, false);
-    if (dtype == RB_BF16) RB_RECUR(bf16, true);
+    if (prep != nullptr && recurrence_chunked(dtype, dk) && max_q_len > rb_recurrence_tile(dk)) return recurrence_chunks(A, form, n_entries, st);
+#define RB_RECUR(TA) \
+    do { if (form == 0) return recurrence_dispatch<TA, 0>(A, n_entries, max_q_len, st); \
+         if (form == 1) return recurrence_dispatch<TA, 1>(A, n_entries, max_q_len, st); \
+         if (form == 3) return recurrence_dispatch<TA, 3>(A, n_entries, max_q_len, st); \
+         return recurrence_dispatch<TA, 2>(A, n_entries, max_q_len, st); } while (0)
+    if (dtype == RB_F32) RB_RECUR(float);
+    if (dtype == RB_BF16) RB_RECUR(bf16);
 #undef RB_RECUR
     RB_REFUSE("recurrence: dtype %d", dtype);
 }

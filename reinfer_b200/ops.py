@@ -39,6 +39,7 @@ def lib():
         except OSError as e:
             raise KernelError(f"cannot load the kernel library {path}: {e}") from None
         _lib.rb_last_error.restype = c_char_p
+        _lib.rb_recurrence_scratch_floats.restype = c_longlong
         if _lib.rb_abi_version() != 1:
             raise KernelError("kernel library has another ABI version")
         if os.environ.get("REINFER_B200_GEMM_SCHEDULE"):
@@ -1705,8 +1706,9 @@ def recurrence(form: str, gate: str, q: torch.Tensor, k: torch.Tensor, v: torch.
     # step's tokens, into a scratch buffer (a decode step, whose captured form has max_q_len 1, never takes it)
     prep = None
     if max_q_len > int(lib().rb_recurrence_tile(c_int(dk))):
-        prep = torch.empty(T * H * int(lib().rb_recurrence_record_floats(c_int(RECURRENCE_FORMS[form]), c_int(dk), c_int(dv))),
-                           dtype=torch.float32, device=q.device)
+        floats = lib().rb_recurrence_scratch_floats(c_int(RECURRENCE_FORMS[form]), c_int(dt(q)), c_int(dk), c_int(dv), c_int(H),
+                                                    c_int(T), c_int(n_entries))
+        prep = torch.empty(floats, dtype=torch.float32, device=q.device)
     _check(lib().rb_recurrence(c_int(RECURRENCE_FORMS[form]), c_int(RECURRENCE_GATES[gate]), c_int(dt(q)),
                                _p(q), ld(q), _p(k), ld(k), _p(v), ld(v), _p(z), ld(z), _p(z_bias), c_int(int(gate_per_head)),
                                _p(a_pre), ld(a_pre), _p(a_bias), _p(b_pre), ld(b_pre), _p(rate), _p(bonus),
