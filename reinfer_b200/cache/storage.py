@@ -13,10 +13,11 @@ page index: crates/cuda/src/decode.rs:664-698.)
 """
 from __future__ import annotations
 
-from typing import Dict, List
+from typing import Dict, List, Sequence
 
 import torch
 
+from .. import ops
 from .manager import CacheManager
 
 
@@ -57,6 +58,9 @@ class CacheStorage:
         for name, spec in manager.states.items():
             self.layer_state[name] = make(spec)
         self.inert_slot = manager.max_seqs
+        tensors = self.state_tensors()
+        # where the rows of these tensors lie, for the kernel that sets a request's to zero
+        self._zero_rows = ops.zero_slots_table(tensors, self.device) if tensors else None
         # the request slots' own rows (as many, plus nobody's): the token last drawn for the request, the sampler's
         # record (parameters, seed, count of draws: csrc/sampler.cu RbSampleParams) and its ring of recent tokens.
         # The sampler kernel reads and writes them; the host writes a row when a request is admitted.
@@ -75,10 +79,10 @@ class CacheStorage:
                 bad += [f"{name}: {which}" for name, t in zip(g.layers, touched) if t]
         return bad
 
-    def zero_slot(self, slot: int) -> None:
+    def zero_slots(self, slots: Sequence[int]) -> None:
         """A fixed-size state starts at zero when its request is admitted."""
-        for t in self.state_tensors():
-            t[slot].zero_()
+        if self._zero_rows is not None and slots:
+            ops.zero_slots(*self._zero_rows, slots)
 
     def state_tensors(self) -> List[torch.Tensor]:
         out: List[torch.Tensor] = []

@@ -358,10 +358,10 @@ class Engine:
         if need > cm.free_pages():
             raise OutOfPages(f"the step needs {need} more pages, {cm.free_pages()} are free")
         self._undo = cm.snapshot([e.request_id for e in entries])     # from here on the manager changes
-        for e in new:
-            slot = cm.admit(e.request_id)
-            self.storage.zero_slot(slot)
-            if self.on_admit is not None:
+        admitted = [cm.admit(e.request_id) for e in new]
+        self.storage.zero_slots(admitted)
+        if self.on_admit is not None:
+            for e, slot in zip(new, admitted):
                 self.on_admit(e.request_id, slot)
         # decode entries first, each kind in the order given
         order = sorted(range(len(entries)), key=lambda i: (len(entries[i].tokens) != 1, i))

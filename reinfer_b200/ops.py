@@ -211,6 +211,18 @@ def keep_last_rows(rows: torch.Tensor, state: torch.Tensor, cu_q: torch.Tensor, 
     _check(lib().rb_keep_last_rows(_p(rows), _p(state), c_longlong(size), _p(cu_q), _p(entry_slot), c_int(n_entries), _stream()), "keep_last_rows")
 
 
+def zero_slots_table(tensors, device) -> tuple:
+    """For zero_slots: where the rows of state tensors [slots, ...] lie (their owner keeps them alive as long as the table)."""
+    _need(all(t.is_contiguous() for t in tensors), "zero_slots: contiguous tensors")
+    rows = [(t.data_ptr(), t[0].numel() * t.element_size()) for t in tensors]
+    return torch.tensor(rows, dtype=torch.int64).to(device), max(b for _, b in rows)
+
+
+def zero_slots(table: torch.Tensor, largest: int, slots) -> None:
+    """Row `slot` of every tensor of the table <- 0, for every slot; one launch for up to 64 of them."""
+    _check(lib().rb_zero_slots(_p(table), c_int(table.shape[0]), c_longlong(largest), (c_int * len(slots))(*slots), c_int(len(slots)), _stream()), "zero_slots")
+
+
 def token_shift(h: torch.Tensor, state: torch.Tensor, mu: torch.Tensor, ctx) -> torch.Tensor:
     """[streams, T, C]: h + (h' - h) * mu[s] for every stream s, h' the row of the request's token before (from its slot's row of
     `state` [slots, C] for a portion's first token); the slots' rows move on to the portions' last tokens.  h [T, C] and state
