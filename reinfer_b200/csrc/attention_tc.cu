@@ -3,41 +3,38 @@
 // The formulas are the reference's attention (crates/cuda/kernels/dense_kernels.cu:173-231: scores, causal
 // mask, softmax in float, weighted sum of the values), tiled as flash attention.  A CTA owns 256 query rows: two
 // row tiles A and B of 128 rows each (a row = a token x one of the Gc grouped query heads of one kv head; tile B
-// holds the tokens after tile A's), and walks the request's keys in tiles of 128.  Both row tiles use every key
+// holds the tokens after tile A's), and walks the request's keys in tiles of 64.  Both row tiles use every key
 // tile that comes in, so a key tile is fetched once for 256 rows.  For every key tile j and row tile t
-//     S_t = Q_t K^T        tcgen05.mma, 128 x 128 x 128, operands in shared memory, S in tensor memory
+//     S_t = Q_t K^T        tcgen05.mma, 128 x 64 x 128, operands in shared memory, S in tensor memory (two buffers a row tile)
 //     P_t = exp2(S_t - m)  128 threads, one row each (tcgen05.ld gives a thread its whole row: the row maximum and
-//                          sum need no shuffles), 64 keys at a time, P rounded to bfloat16 into shared memory (a buffer
-//                          per half of the keys and row tile)
-//     O_t += P_t V         tcgen05.mma, 128 x 128 x 64 per half, accumulated in tensor memory over all key tiles: P and O are
+//                          sum need no shuffles), P rounded to bfloat16 and written back to tensor memory, over the scores
+//     O_t += P_t V         tcgen05.mma, 128 x 128 x 64, P from tensor memory, accumulated there over all key tiles: P and O are
 //                          scaled to a maximum that follows the true one only when it rose by more than 2^8 (then the
 //                          row's thread rescales its lane of O in tensor memory, which is rare), so the rows read O once
-// Warp 0 feeds key/value tiles by TMA, 64 keys at a time: ONE request brings the keys (or the values) of a page for this kv
+// Warp 0 feeds key and value tiles by TMA into a ring of four each: ONE request brings the keys (or the values) of a page for this kv
 // head, laid out as [8-key group][64-dim half][8 keys][64 dims] whatever the page size is (the 5-D map of runtime.cu).  Warp 1
-// allocates tensor memory and issues the scores of tile A, warp 3 those of tile B, warp 2 the weighted sums; warps 4-7 are the rows of tile A,
-// warps 8-11 the rows of tile B.  Q [rows][d], K [keys][d] and P [rows][keys] are K-major operands; V [keys][d] is
+// allocates tensor memory and issues the products of tile A, warp 3 those of tile B; warps 4-7 are the rows of tile A,
+// warps 8-11 the rows of tile B.  Q [rows][d] and K [keys][d] are K-major operands; V [keys][d] is
 // used as it lands, as an MN-major operand (instruction descriptor bit 16; in the shared-memory descriptor the
 // leading offset steps to the second 64 dims, the stride offset to the next 8 keys) - nothing is transposed.
 //
-// What runs ahead of what.  A hand-over through an mbarrier that a tcgen05.commit arrives at costs well over a
-// thousand clocks from one side's last instruction to the other side's first.  So no such hand-over may lie on the rows' path
-// from one key tile to the next.  The rows take all 128 scores into registers at once and say so before they exponentiate:
-// the scores of tile j+1 are issued then and stand ready when the rows come back; the weighted sums have their own issuer
-// and nothing but the row's last read of O and the reuse of a P buffer a tile later waits for them.  Shared memory has no
-// room for a third tile of keys, so what waits for what decides: keys have slots of their own, refilled as soon as the scores
-// that read them are there, a tile ahead of their use; values are refilled behind their product and needed half a tile later.
+// What runs ahead of what.  The scores of tile j + 2 go into the columns that P of tile j lay in: their product is issued right behind
+// the weighted sum that reads P, by the same warp, and runs behind it; the rows meanwhile work on tile j + 1 in the other buffer.  So no
+// hand-over lies on the rows' path from one key tile to the next.  P does not pass through shared memory: with P there, its
+// writes, the products' two reads of every operand and the copies wanted 3,070 cycles of shared memory per 128 keys, at 128 bytes a
+// cycle, where the tensor cores want 2,048.
 //
-// What bounds a key tile now: a row warp's own work.  Of the about 3,900 cycles that a tile takes it is at work 3,750: 2,530 in the
-// exponentials' passes, about 1,200 outside of them (scores into registers, edge tests, fences and arrivals); it waits 220 for
-// scores and 230 for its P buffer.  (-DRB_TIMELINE: lane 0 of every warp adds up its waits and its work.)  The special-function
-// units have 2,048 cycles of exponentials a tile and the tensor cores 2,048 of products, about half of the time each.
-// 2,048 tokens behind 14,336 others, 32 query over 8 kv heads: 525 us (980 TFLOP/s); tiles of 64 keys with two score buffers
-// took 663, 128 keys in one ring of keys and values 642 (128 keys alone 1 % more than 663: what that gave was the options' code out
-// of the loop and one copy of the exponentials').
+// What bounds it (-DRB_TIMELINE, cycles per 64 keys; 2,048 tokens behind 14,336 others, 32 query over 8 kv heads): a row warp works
+// 1,480, of them 1,230 in the exponentials (the special-function unit needs 1,024 for the two row warps of a scheduler), and waits 220
+// for scores; the tensor pipe is busy 1,280 (a 128 x 64 product of scores reads 6 KB of shared memory, 48 cycles for 32 of arithmetic).
+// 473 us (1,090 TFLOP/s); with P in shared memory, scores of 128 keys and a third issuing warp for the weighted sums 526.  256 CTAs of
+// equal length are 1.73 rounds over 148 SMs, which costs another seventh.  Measured beside it: products of 128 x 128 scores with P over
+// them, whose rows wait for product, hand-over and product again (664 us); one score buffer and two of P beside it (554); barriers of
+// keys and values looked at only when they are needed (500: a wait costs an issuer 135 cycles however long ago the bytes came).
 // Scaling, sums and maxima are packed or three-input instructions, and the code of the options is in instantiations of its
 // own, for the rows' loop has to fit the instruction cache: with all options in it, a fifth of the rows' stalls were
-// instruction fetches.  Built, measured, left out: two threads per row (the row's maximum agreed through shared memory: 11 %
-// slower); a part of the exponentials as a cubic on the FMA pipe (8 to 16 % slower); P rounded by integer instructions.
+// instruction fetches.  Built, measured, left out before P moved: two threads per row (the row's maximum agreed through shared memory:
+// 11 % slower); a part of the exponentials as a cubic on the FMA pipe (8 to 16 % slower); P rounded by integer instructions.
 // Registers follow the roles (setmaxnreg): 64 for the control warps, 216 for the rows - what the control warps give up
 // (128 threads x 104) must cover what the rows take (256 threads x 48), for the registers come from the CTA's own
 // allocation (384 x 168) and a request for more than it holds waits for ever.
@@ -50,21 +47,24 @@
 #include "sm100.cuh"
 #include <stdlib.h>
 
-#define FC_BN 64                              // keys per half tile: what one weighted sum takes
-#define FC_KEYS (2 * FC_BN)                   // keys per tile: what one product of scores takes
+#define FC_BN 64                              // keys per key tile
 #define FC_ROWS 128                           // query rows per row tile
 #define FC_TILES 2                            // row tiles per CTA
 #define FC_D 128
-#define FC_THREADS 384                        // a control group (TMA, scores of tile A, weighted sums, scores of tile B) and two groups of four row warps
-#define FC_SLOTS 6                            // half tiles: keys of even tiles in slots 0, 1, of odd tiles in 2, 3; values in 4, 5
-#define FC_KSLOT(tile) (((tile) & 1) * 2)
-#define FC_VSLOT(half) (4 + ((half) & 1))
+#define FC_THREADS 384                        // a control group (TMA, products of tile A, -, products of tile B) and two groups of four row warps
+#define FC_RING 4                             // key tiles, and value tiles, in shared memory
+#define FC_SLOTS (2 * FC_RING)                // keys in slots 0 .., values behind them
+#define FC_KSLOT(tile) ((tile) % FC_RING)
+#define FC_VSLOT(tile) (FC_RING + (tile) % FC_RING)
+#define FC_PHASE(tile) ((uint32_t)(((tile) / FC_RING) & 1))
 #define FC_KV_BYTES (FC_BN * 256)             // a slot: 64 keys (or values) x 256 bytes, as 8 groups of [2 halves][8 keys][128 bytes]
 #define FC_GROUP 2048                         // bytes from one 8-key group to the next
 #define FC_HALF 1024                          // bytes from a group's first 64 dims to its second
-#define FC_QHALF (FC_ROWS * 128)              // 128 rows x 128 bytes: one 64-column half of a Q tile, or one P buffer
+#define FC_QHALF (FC_ROWS * 128)              // 128 rows x 128 bytes: one 64-column half of a Q tile
 #define FC_RESCALE 8.0f                       // O is brought to a new maximum only when it rose by more than this (log2)
-#define FC_TMEM_COLS 512                      // S_A: columns 0..127; S_B 128..255; O_A 256..383; O_B 384..511
+#define FC_TMEM_COLS 512                      // S_A: columns 0..63 and 64..127, P_A in the first half of either; S_B 128..255; O_A 256..383; O_B 384..511
+#define FC_S(t, tile) ((uint32_t)((t) * 2 * FC_BN + ((tile) & 1) * FC_BN))
+#define FC_O(t) ((uint32_t)(FC_TILES * 2 * FC_BN + (t) * FC_D))
 
 struct FcArgs {
     const bf16* q;
@@ -100,8 +100,9 @@ struct FcArgs {
 
 struct FcShared {
     unsigned long long full[FC_SLOTS];
-    unsigned long long empty[FC_SLOTS];
-    unsigned long long s_full[FC_TILES], s_free[FC_TILES], p_full[FC_TILES][2], o_full[FC_TILES][2];
+    unsigned long long done[FC_RING];                              // [i % FC_RING]: either issuer's scores of tile i and weighted sum of tile i - 2
+    unsigned long long s_full[FC_TILES][2], p_full[FC_TILES][2];
+    unsigned long long o_full[FC_TILES][2];                        // the weighted sums up to the last tile but one; up to the last (one use each)
     int uses[FC_SLOTS];                                            // copies issued into each slot
     uint32_t tmem_base;
     int abort_flag;
@@ -115,6 +116,15 @@ __device__ __forceinline__ uint32_t fc_off(int row, int c, int half_bytes) {
 // the same for a key/value tile as the 5-D map lays it out: [8-key group][half][8 keys][128 bytes]
 __device__ __forceinline__ uint32_t fc_kv_off(int key, int c) {
     return (uint32_t)((key >> 3) * FC_GROUP + (c >> 3) * FC_HALF + (key & 7) * 128 + (((c & 7) ^ (key & 7)) << 4));
+}
+// D += A B with A in tensor memory (a lane a row, two 16-bit elements along K a column); see fc_mma_ss.
+__device__ __forceinline__ void fc_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, uint32_t lead) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
 }
 // Sixteen 32-bit columns of this warp's 32 lanes back into tensor memory (the counterpart of tc_ld16).
 __device__ __forceinline__ void fc_st16(uint32_t taddr, const uint32_t* r) {
@@ -245,25 +255,23 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* stages = smem;                                  // [FC_SLOTS]
     unsigned char* sQ = stages + FC_SLOTS * FC_KV_BYTES;           // [row tile][two halves of [128 rows][64 dims]]
-    unsigned char* sP = sQ + FC_TILES * 2 * FC_QHALF;              // [row tile][buffer][128 rows][64 keys]
-    FcShared* sh = (FcShared*)(sP + FC_TILES * 2 * FC_QHALF);
-    const uint32_t stages_u = smem_u32(stages), sQ_u = smem_u32(sQ), sP_u = smem_u32(sP);
+    FcShared* sh = (FcShared*)(sQ + FC_TILES * 2 * FC_QHALF);
+    const uint32_t stages_u = smem_u32(stages), sQ_u = smem_u32(sQ);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     volatile int* abort_flag = &sh->abort_flag;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < FC_SLOTS; ++s) {
             mbar_init(smem_u32(&sh->full[s]), 1);
-            mbar_init(smem_u32(&sh->empty[s]), 2);                 // the issuers' commits: scores (keys) or weighted sums (values) of either row tile done
             sh->uses[s] = 0;
         }
+        for (int s = 0; s < FC_RING; ++s) mbar_init(smem_u32(&sh->done[s]), 2);
         for (int t = 0; t < FC_TILES; ++t) {
-            mbar_init(smem_u32(&sh->s_full[t]), 1);
-            mbar_init(smem_u32(&sh->s_free[t]), 4);                // one arrival per row warp: the scores are in registers
             for (int b = 0; b < 2; ++b) {
+                mbar_init(smem_u32(&sh->s_full[t][b]), 1);
                 mbar_init(smem_u32(&sh->p_full[t][b]), 4);         // one arrival per row warp: P is written
-                mbar_init(smem_u32(&sh->o_full[t][b]), 1);
             }
+            for (int b = 0; b < 2; ++b) mbar_init(smem_u32(&sh->o_full[t][b]), 1);
         }
         sh->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -293,7 +301,7 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
         tile -= nt;
     }
     const bool none = e >= a.first_entry + a.n_entries;            // uniform: a CTA beyond the last entry
-    int n_halves = 0, q0 = 0, n_tok = 0, kv_end = 0, start_pos = 0, tok_base = 0, t_begin = 0, head0 = 0, kh = 0;
+    int n_tiles = 0, q0 = 0, n_tok = 0, kv_end = 0, start_pos = 0, tok_base = 0, t_begin = 0, head0 = 0, kh = 0;
     const int* bt = a.block_table;
     if (!none) {
         q0 = tile * tpc;
@@ -308,7 +316,7 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
         int lo_min = a.window > 0 ? max(0, pos_min - a.window + 1) : 0;
         if (a.chunk > 0) lo_min = max(lo_min, pos_min / a.chunk * a.chunk);
         t_begin = lo_min / FC_BN;
-        n_halves = pos_max / FC_BN + 1 - t_begin;
+        n_tiles = pos_max / FC_BN + 1 - t_begin;
         // Q rows (row r of the CTA = token r / Gc, grouped head r % Gc; rows 128.. are tile B) into the swizzled K-major layout
         for (int i = threadIdx.x; i < n_tok * a.Gc * (FC_D / 8); i += FC_THREADS) {
             const int row = i / (FC_D / 8), c = i % (FC_D / 8);
@@ -327,16 +335,12 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
     }
     __syncthreads();
 
-    const int n_tiles = (n_halves + 1) / 2;
     [[maybe_unused]] long long fc_acc[7] = {0, 0, 0, 0, 0, 0, 0};
     if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");           // the control group gives registers up ...
     if (warp == 0) {
-        // ---- producer: the keys of tile i + 1 go out before the values of tile i.  A tile's keys find their slots free as soon as
-        // the scores of two tiles before are there, a tile ahead of their use; values wait for the product of the tile
-        // before, and are needed half a tile after its rows began.  (One ring of six slots in the order of use had the
-        // keys wait for that product too: the rows then waited 800 of 4,700 cycles for their scores.)
-        // Block-table entries 32 at a time, in windows that begin at multiples of 32, which a half's pages (eight at most) never
+        // ---- producer: keys 0, keys 1, values 0, keys 2, values 1, ... each into its ring.
+        // Block-table entries 32 at a time, in windows that begin at multiples of 32, which a tile's pages (eight at most) never
         // cross: the window of the keys, the one before it (values lie up to 24 pages behind the keys that went out before them), and
         // the one after it, asked for a window ahead of its use.
         const int box_keys = min(a.page_size, FC_BN);              // keys that one request brings
@@ -346,26 +350,27 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
         int window = ((t_begin * FC_BN) >> a.page_shift) >> 5;
         int before = -1, here = entries(window), after = entries(window + 1);
         bool ok = true;
-        for (int step = 0; step < 2 * n_tiles + 1 && ok; ++step) { // keys 0; keys 1, values 0; keys 2, values 1; ...
-            const int values = step > 0 && !(step & 1), tile = values ? step / 2 - 1 : (step + 1) / 2;
-            if (tile >= n_tiles) continue;
-#pragma unroll 1
-            for (int half = 2 * tile; half < min(2 * tile + 2, n_halves); ++half) {
-                const int k0 = (t_begin + half) * FC_BN;
-                const int own = (k0 >> a.page_shift) >> 5;         // (a half is at most eight pages behind the last: one window further)
+        for (int step = 0; step < 2 * n_tiles + 2 && ok; ++step) {
+            const int values = step >= 2 && !(step & 1), tile = values ? step / 2 - 1 : (step + 1) / 2;
+            if (tile < n_tiles) {
+                const int k0 = (t_begin + tile) * FC_BN;
+                const int own = (k0 >> a.page_shift) >> 5;         // (a tile is at most eight pages behind the last: one window further)
                 if (own > window) { before = here; here = after; after = entries(++window + 1); }
-                const int s = values ? FC_VSLOT(half) : FC_KSLOT(tile) + (half & 1), use = values ? tile : tile >> 1;
+                const int s = values ? FC_VSLOT(tile) : FC_KSLOT(tile), use = tile / FC_RING;
                 const uint32_t full = smem_u32(&sh->full[s]);
                 const uint32_t dst0 = stages_u + s * FC_KV_BYTES;
-                // A lane for each page of this half, which makes the page's request itself, all in one instruction.  (Lane 0 making them
+                // A lane for each page of this tile, which makes the page's request itself, all in one instruction.  (Lane 0 making them
                 // one after the other took some 200 cycles a request: 16 of them per 64 keys and values in pages of 8 keys are more than
-                // the 2,000 that the products and rows need.  32 query over 8 kv heads, 2,048 tokens behind 14,336 others:
-                // pages of 8 keys 951 -> 618 us, of 16 652 -> 526, of 64 531 -> 525.)
+                // the products and rows need.  32 query over 8 kv heads, 2,048 tokens behind 14,336 others: pages of 8 keys 548 us, of
+                // 16 and 64 473; one after the other 951, 652 and 531 with P in shared memory, 618, 526 and 525 in one instruction.)
                 const int my_key = k0 + lane * box_keys;
                 const int my_page = __shfl_sync(0xffffffffu, own == window ? here : before, (my_key >> a.page_shift) & 31);
                 const uint32_t there = __ballot_sync(0xffffffffu, lane < subs && my_key < kv_end && my_page >= 0);
                 const int my_index = (my_page * 2 + values) * a.KH + kh, grp = (k0 & (a.page_size - 1)) >> 3;
-                { FC_T0(); if (use && !fc_wait(smem_u32(&sh->empty[s]), (uint32_t)((use & 1) ^ 1), abort_flag, 11)) { ok = false; break; } FC_ADD(0); }
+                // What was here before has been used: keys by the scores of the tile FC_RING before, values by that tile's weighted sum,
+                // which goes with the scores two tiles on.
+                const int user = values ? tile - FC_RING + 2 : tile - FC_RING;
+                { FC_T0(); if (use && !fc_wait(smem_u32(&sh->done[user % FC_RING]), FC_PHASE(user), abort_flag, 11)) { ok = false; break; } FC_ADD(0); }
                 FC_T0();
                 mbar_expect_tx_lead(full, (uint32_t)(__popc(there) * box_keys * 256), lead);
                 __syncwarp();                                      // the barrier expects the bytes before the first of them can arrive
@@ -376,25 +381,25 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
         }
         FC_FLUSH(n_tiles);
     } else if (warp == 1 || warp == 3) {
-        // ---- issuers of the scores, one warp per row tile: every lane runs the loop, lane 0's instructions take effect
-        // S_t(i) = Q_t K(i)^T over the 128 keys of a tile, as soon as the keys have landed and the rows have taken the
-        // scores of the tile before out of tensor memory: the scores run ahead of the rows, whatever the products P V
-        // are doing.  d = 128 is two 64-column halves of four 16-wide steps each; the keys' 8-row groups lie 2,048 bytes
-        // apart (through both slots), their second half 1,024 bytes on.  (One warp for both row tiles had twice the
-        // products and commits to issue, about 65 cycles each: more than the products take to run.)
+        // ---- issuers, one warp per row tile: every lane runs the loop, lane 0's instructions take effect
+        // O_t += P_t(i) V(i) once the rows have written P, then S_t(i + 2) = Q_t K(i + 2)^T into the columns that P(i) lay in: one warp
+        // issues both, and the products of one issuer run in the order they were issued in, so nothing waits between them.  d =
+        // 128 is two 64-column halves of four 16-wide steps each; the keys' 8-row groups lie 2,048 bytes apart, their second half
+        // 1,024 bytes on.  V [keys][d] as it lies in its slot is an MN-major operand: a key's 64 dims (128 bytes) contiguous, keys
+        // 128 bytes apart, groups of 8 keys 2,048 bytes apart (SBO), the second 64 dims 1,024 bytes on (LBO); an MMA takes 16 keys =
+        // two groups of V and eight columns of P.  (One warp for both row tiles had twice the products and commits to issue, about 65
+        // cycles each: more than the products take to run.)
         const uint32_t lead = lane == 0 ? 1u : 0u;
         const int t = warp == 1 ? 0 : 1;
-        constexpr uint32_t idesc_s = make_idesc(FC_KEYS);
+        constexpr uint32_t idesc_s = make_idesc(FC_BN), idesc_mn = make_idesc(FC_D) | (1u << 16);      // B of the weighted sum is MN-major
         const uint64_t dq0 = make_smem_desc(sQ_u + (t * 2) * FC_QHALF), dq1 = make_smem_desc(sQ_u + (t * 2 + 1) * FC_QHALF);
-        for (int i = 0; i < n_tiles; ++i) {
+        // Whether keys and values have landed is asked while the products before theirs are issued: a wait costs over a hundred
+        // cycles however long ago the bytes came, and the tensor pipe runs dry meanwhile.
+        bool keys_there = false, values_there = false;
+        auto scores = [&](int i) -> bool {
             const int s = FC_KSLOT(i);
-            const bool both = 2 * i + 1 < n_halves;                // (a missing half's scores are never read)
-            const uint32_t par = (uint32_t)((i >> 1) & 1);
-            { FC_T0(); if (!fc_wait(smem_u32(&sh->full[s]), par, abort_flag, 12)) break;
-              if (both && !fc_wait(smem_u32(&sh->full[s + 1]), par, abort_flag, 12)) break; FC_ADD(0); }
-            { FC_T0(); if (i >= 1 && !fc_wait(smem_u32(&sh->s_free[t]), (uint32_t)((i & 1) ^ 1), abort_flag, 20)) break; FC_ADD(1); }
+            { FC_T0(); if (!keys_there && !fc_wait(smem_u32(&sh->full[s]), FC_PHASE(i), abort_flag, 12)) return false; FC_ADD(0); }
             FC_T0();
-            tc_fence_after();
             const uint32_t sK = stages_u + s * FC_KV_BYTES;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -402,40 +407,39 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
                 const uint64_t dk = make_smem_desc_lbo_sbo(sK + h * FC_HALF, 16, FC_GROUP);
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
-                    fc_mma_ss(tmem + (uint32_t)(t * FC_KEYS), dq + (uint64_t)(k * 2), dk + (uint64_t)(k * 2), idesc_s, (h | k) != 0, lead);
+                    fc_mma_ss(tmem + FC_S(t, i), dq + (uint64_t)(k * 2), dk + (uint64_t)(k * 2), idesc_s, (h | k) != 0, lead);
             }
-            fc_commit_lead(smem_u32(&sh->s_full[t]), lead);
-            fc_commit_lead(smem_u32(&sh->empty[s]), lead);         // the keys are read once these MMAs are done
-            if (both) fc_commit_lead(smem_u32(&sh->empty[s + 1]), lead);
+            fc_commit_lead(smem_u32(&sh->s_full[t][i & 1]), lead);
             FC_ADD(2);
-        }
-        FC_FLUSH(n_tiles);
-    } else if (warp == 2) {
-        // ---- issuer of the weighted sums: O_t += P_t V once the rows of tile t have written P -----------------------
-        const uint32_t lead = lane == 0 ? 1u : 0u;
-        constexpr uint32_t idesc_mn = make_idesc(FC_D) | (1u << 16);           // B is MN-major
-        bool ok = true;
-        for (int ht = 0; ht < n_halves && ok; ++ht) {
-            const int s = FC_VSLOT(ht);
-            // V [keys][d] as it lies in its slot is an MN-major operand: a key's 64 dims (128 bytes) contiguous, keys
-            // 128 bytes apart, groups of 8 keys 2,048 bytes apart (SBO), the second 64 dims 1,024 bytes on (LBO); an
-            // MMA takes 16 keys = two groups.
+            return true;
+        };
+        auto done = [&](int i) { fc_commit_lead(smem_u32(&sh->done[i % FC_RING]), lead); };
+        bool ok = n_tiles < 1 || scores(0);
+        if (ok) done(0);
+        ok = ok && (n_tiles < 2 || scores(1));
+        if (ok) done(1);
+        for (int i = 0; i < n_tiles && ok; ++i) {
+            const int s = FC_VSLOT(i);
+            const uint32_t par = (uint32_t)((i >> 1) & 1);
+            { FC_T0(); if (!values_there && !fc_wait(smem_u32(&sh->full[s]), FC_PHASE(i), abort_flag, 21)) break; FC_ADD(1); }
+            { FC_T0(); if (!fc_wait(smem_u32(&sh->p_full[t][i & 1]), par, abort_flag, 13)) break; FC_ADD(3); }
+            // the request's last values: rows of tile A have set what lies behind them to zero before they said that P is there
+            if (t == 1 && (t_begin + i + 1) * FC_BN > kv_end && !fc_wait(smem_u32(&sh->p_full[0][i & 1]), par, abort_flag, 20)) break;
+            FC_T0();
+            tc_fence_after();
             const uint64_t dv = make_smem_desc_lbo_sbo(stages_u + s * FC_KV_BYTES, FC_HALF, FC_GROUP);
-            { FC_T0(); if (!fc_wait(smem_u32(&sh->full[s]), (uint32_t)((ht >> 1) & 1), abort_flag, 21)) break; FC_ADD(1); }
 #pragma unroll
-            for (int t = 0; t < FC_TILES; ++t) {
-                { FC_T0(); if (!fc_wait(smem_u32(&sh->p_full[t][ht & 1]), (ht >> 1) & 1, abort_flag, 13)) { ok = false; break; } FC_ADD(0); }
-                FC_T0();
-                tc_fence_after();
-                const uint64_t dp = make_smem_desc(sP_u + (t * 2 + (ht & 1)) * FC_QHALF);
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    fc_mma_ss(tmem + (uint32_t)(FC_TILES * FC_KEYS + t * FC_D), dp + (uint64_t)(k * 2),
-                              dv + (uint64_t)(k * ((2 * FC_GROUP) >> 4)), idesc_mn, (ht > 0) || k != 0, lead);
-                fc_commit_lead(smem_u32(&sh->o_full[t][ht & 1]), lead);
-                fc_commit_lead(smem_u32(&sh->empty[s]), lead);     // the values of this slot are read once these are done (for either row tile)
-                FC_ADD(2);
+            for (int k = 0; k < 4; ++k) {
+                fc_mma_ts(tmem + FC_O(t), tmem + FC_S(t, i) + (uint32_t)(k * 8), dv + (uint64_t)(k * ((2 * FC_GROUP) >> 4)), idesc_mn, (i > 0) || k != 0, lead);
+                if (k == 0) {
+                    keys_there = i + 2 < n_tiles && mbar_test(smem_u32(&sh->full[FC_KSLOT(i + 2)]), FC_PHASE(i + 2));
+                    values_there = i + 1 < n_tiles && mbar_test(smem_u32(&sh->full[FC_VSLOT(i + 1)]), FC_PHASE(i + 1));
+                }
             }
+            if (i + 2 >= n_tiles) fc_commit_lead(smem_u32(&sh->o_full[t][i + 1 == n_tiles]), lead);
+            FC_ADD(2);
+            if (i + 2 < n_tiles && !scores(i + 2)) break;
+            done(i + 2);
         }
         FC_FLUSH(n_tiles);
     }
@@ -462,33 +466,24 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
         // FC_RESCALE, so that O can stay in tensor memory and be accumulated by the MMA itself); l: the sum in that scale
         float m = -INFINITY, l = 0.0f;
         const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
-        const uint32_t o_col = (uint32_t)(FC_TILES * FC_KEYS + t * FC_D);
+        const uint32_t o_col = FC_O(t);
         bool ok = true;
         for (int it = 0; it < n_tiles && ok; ++it) {
-            // S: this row's 128 scores in one go (one wait for tensor memory); then the next tile's may come
-            uint32_t s_all[FC_KEYS];
-            { FC_T0(); if (!fc_wait(smem_u32(&sh->s_full[t]), (uint32_t)(it & 1), abort_flag, 15)) { ok = false; break; } FC_ADD(0); }
+            // S: this row's 64 scores in one go (one wait for tensor memory)
+            const int b = it & 1, k0 = (t_begin + it) * FC_BN;
+            uint32_t sr[FC_BN];
+            { FC_T0(); if (!fc_wait(smem_u32(&sh->s_full[t][b]), (uint32_t)((it >> 1) & 1), abort_flag, 15)) { ok = false; break; } FC_ADD(0); }
 #ifdef RB_TIMELINE
             const long long fc_tile0 = clock64();
 #endif
             tc_fence_after();
 #pragma unroll
-            for (int c = 0; c < FC_KEYS / 16; ++c) tc_ld16(lane_base + (uint32_t)(t * FC_KEYS + c * 16), s_all + c * 16);
+            for (int c = 0; c < FC_BN / 16; ++c) tc_ld16(lane_base + FC_S(t, it) + (uint32_t)(c * 16), sr + c * 16);
             tc_ld_wait();
 #ifdef RB_TIMELINE
             fc_acc[1] += clock64() - fc_tile0;
 #endif
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&sh->s_free[t]));
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {                          // 64 keys at a time: P, and the weighted sum that may begin on it
-            if (2 * it + b >= n_halves) break;
-            uint32_t* sr = s_all + b * FC_BN;
-            const int k0 = (t_begin + 2 * it + b) * FC_BN;
-            const uint32_t par = (uint32_t)(it & 1);
             const bool edge = k0 + FC_BN - 1 > pos || k0 < lo;     // these keys cross this row's causal edge or window
-            const bool begins = it == 0 && b == 0;
             if ((OPTIONS & FC_CAP) && a.cap_raw > 0.0f) {
                 // tanh z = 1 - 2 / (e^(2z) + 1): one exponential and one reciprocal of the special-function unit, exact
                 // at both ends (e = inf gives 1, e = 0 gives -1); the error is an absolute 2^-23 or so of the cap
@@ -524,19 +519,13 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
                     if (key < lo || key > pos) sr[j] = 0xff800000u;            // -inf
                 }
             }
-            // this P buffer was read by the product of the key tile before, which must be done before it is written again
-            if (it >= 1) {
-                FC_T0();
-                if (!fc_wait(smem_u32(&sh->o_full[t][b]), par ^ 1, abort_flag, 16)) { ok = false; break; }
-                FC_ADD(2);
-            }
             if (t == 0 && k0 + FC_BN > kv_end) {
                 // the request's last keys: slots of its last page beyond its length hold foreign data - the values
                 // there are zeroed before the tensor core multiplies them (by P = 0, but 0 x NaN is NaN).  The rows of
-                // tile A do it; the product of tile B is issued behind A's, so it sees the zeros too.  (Behind the wait above: the
-                // product of the tile before has then read this slot, so its barrier cannot be two phases behind.)
-                const int s = FC_VSLOT(b);
-                if (!fc_wait(smem_u32(&sh->full[s]), par, abort_flag, 14)) { ok = false; break; }
+                // tile A do it, and the issuer of tile B's product waits for them.  (Scores of this tile stand behind the product of the
+                // tile two before, so this slot's barrier cannot be two phases behind.)
+                const int s = FC_VSLOT(it);
+                if (!fc_wait(smem_u32(&sh->full[s]), FC_PHASE(it), abort_flag, 14)) { ok = false; break; }
                 unsigned char* sV = stages + s * FC_KV_BYTES;
                 for (int i = row; i < FC_BN * 16; i += FC_ROWS) {
                     const int r = i / 16, c = i % 16;
@@ -544,9 +533,9 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the zeros, before the tensor core reads the values
             }
-            unsigned char* sPb = sP + (t * 2 + b) * FC_QHALF;
-            // P = 2^(S * scale - base), rounded to bfloat16, into the buffer; its row sum; and, beside the exponentials (nothing
+            // P = 2^(S * scale - base), rounded to bfloat16, two a register; its row sum; and, beside the exponentials (nothing
             // here waits for it), the maximum of the raw scores in `top`
+            uint32_t pr[FC_BN / 2];
             float top = -INFINITY;
             auto emit = [&](float base) -> float {
                 unsigned long long sum2[2] = {0ull, 0ull};             // four running sums, packed in pairs
@@ -564,9 +553,8 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
                         p[j + 1] = fc_ex2(p[j + 1]);
                         sum2[(j >> 1) & 1] = fc_add2(sum2[(j >> 1) & 1], fc_pair(p[j], p[j + 1]));
                     }
-                    uint4 pk;
-                    pk.x = fc_pack(p[0], p[1]); pk.y = fc_pack(p[2], p[3]); pk.z = fc_pack(p[4], p[5]); pk.w = fc_pack(p[6], p[7]);
-                    *reinterpret_cast<uint4*>(sPb + fc_off(row, c, 0)) = pk;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) pr[c * 4 + j] = fc_pack(p[2 * j], p[2 * j + 1]);
                 }
                 top = fmaxf(fc_max3(mx4[0], mx4[1], mx4[2]), mx4[3]);
                 float s0, s1, s2, s3;
@@ -594,10 +582,12 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
                 if (m == -INFINITY) m = mx;
                 else if (moves) { alpha = fc_ex2(m - mx); m = mx; }
                 l *= alpha;
-                if (begins || !__any_sync(0xffffffffu, alpha != 1.0f)) continue;
+                if (it == 0 || !__any_sync(0xffffffffu, alpha != 1.0f)) continue;
                 // rare: O = O * alpha in tensor memory, every lane of the warp with its own factor (1 for most); the
                 // product of the 64 keys before (the last one that can have been issued) must have landed in O first
-                if (!fc_wait(smem_u32(&sh->o_full[t][b ^ 1]), (uint32_t)((b ? it : it - 1) & 1), abort_flag, 18)) { ok = false; break; }
+                // (the next tile's scores, issued behind it, say so; behind the last tile there are none)
+                if (it + 1 < n_tiles ? !fc_wait(smem_u32(&sh->s_full[t][b ^ 1]), (uint32_t)(((it + 1) >> 1) & 1), abort_flag, 18)
+                                     : !fc_wait(smem_u32(&sh->o_full[t][0]), 0u, abort_flag, 16)) { ok = false; break; }
                 tc_fence_after();
 #pragma unroll 1
                 for (int c = 0; c < FC_D / 32; ++c) {
@@ -620,25 +610,22 @@ fa_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const FcArgs a)
 #ifdef RB_TIMELINE
             const long long fc_c6 = clock64();
 #endif
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // P (and zeroed value rows) before the tensor core reads them
-            tc_fence_before();                                     // O (if touched) is written: the product may go on
+            fc_st16(lane_base + FC_S(t, it), pr);                  // over the scores, which are in registers
+            fc_st16(lane_base + FC_S(t, it) + 16u, pr + 16);
+            fc_st_wait();
+            tc_fence_before();                                     // P (and O, if touched) is written: the product may go on
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&sh->p_full[t][b]));
 #ifdef RB_TIMELINE
             fc_acc[6] += clock64() - fc_c6;
 #endif
-            }
 #ifdef RB_TIMELINE
             fc_acc[4] += clock64() - fc_tile0;
 #endif
         }
         FC_FLUSH(n_tiles);
-        // the row of O, once the tile's last products are done (the last one on each of the two barriers)
-        if (ok && n_tiles > 0) {
-            const int last = n_halves - 1;
-            ok = fc_wait(smem_u32(&sh->o_full[t][last & 1]), (uint32_t)((last >> 1) & 1), abort_flag, 17);
-            if (ok && last >= 1) ok = fc_wait(smem_u32(&sh->o_full[t][(last - 1) & 1]), (uint32_t)(((last - 1) >> 1) & 1), abort_flag, 19);
-        }
+        // the row of O, once the last product is done
+        if (ok && n_tiles > 0) ok = fc_wait(smem_u32(&sh->o_full[t][1]), 0u, abort_flag, 17);
         if (ok && n_tiles > 0 && !*abort_flag) {
             // (the loads from tensor memory are the whole warp's: every lane takes part, only live rows store)
             tc_fence_after();
@@ -730,7 +717,7 @@ extern "C" int rb_fa_prefill_tc(const void* q, const void* cache, long long num_
     a.sink = sink; a.gate = gate; a.gate_stride = gate_stride; a.gate_heads = gate_heads;
     CUtensorMap map;
     if (rb_tensor_map_kv_pages(cache, num_pages, KH, page_size, &map)) return -1;
-    constexpr size_t smem = (size_t)FC_SLOTS * FC_KV_BYTES + FC_TILES * 4 * FC_QHALF + sizeof(FcShared) + 1024;
+    constexpr size_t smem = (size_t)FC_SLOTS * FC_KV_BYTES + FC_TILES * 2 * FC_QHALF + sizeof(FcShared) + 1024;
     static_assert(smem <= 232448, "more than the shared memory of an SM");
     if (n_tiles > 65535) RB_REFUSE("attention (tcgen05): %d row tiles in one launch", n_tiles);
     const int options = (softcap > 0.0f ? FC_CAP : 0) | (r1 ? FC_PENALTY : 0) | (bias ? FC_BIAS : 0);
