@@ -1087,9 +1087,9 @@ static int launch_tc_persistent(const CUtensorMap& mw, const CUtensorMap& mx, vo
                      mode, t_tiles, n_tiles, hd, rs);
 }
 
-// The gated pair over 65 .. 128 tokens (a decode step of that many requests): one tile per CTA, 128 tokens (the M
+// The gated pair over 33 .. 128 tokens (a decode step of that many requests): one tile per CTA, 128 tokens (the M
 // operand; rows beyond T are zero-filled by TMA) x 64 gate + 64 up weight rows (the N operand), the whole depth K, three
-// stages of 32 KB - two CTAs fit an SM, and F / 64 CTAs stream the weights (192 at the 8B shape, where 128-row tiles
+// stages of 32 KB (of 24 KB, four, up to 64 tokens) - two CTAs fit an SM, and F / 64 CTAs stream the weights (192 at the 8B shape, where 128-row tiles
 // gave 96 CTAs on 148 SMs with eight products to issue per k-step: 4.4 TB/s).  A lane of the accumulator is a token;
 // its row factor (the deferred RMS norm) multiplies gate and up before the activation.  The weights' first stages are
 // requested before the kernels in front of this one have finished, the tokens after.
@@ -1431,7 +1431,7 @@ static int g_tc_token_lanes = 1;
 extern "C" int rb_set_gemm_token_lanes(int v) { int old = g_tc_token_lanes; g_tc_token_lanes = v ? 1 : 0; return old; }
 
 static int g_tc_gated_stream = 1;
-// The gated pair over 65 .. 128 tokens: 1 = the streaming kernel with a token per lane (64 + 64 weight rows a CTA),
+// The gated pair over 33 .. 128 tokens: 1 = the streaming kernel with a token per lane (64 + 64 weight rows a CTA),
 // 0 = the kernel with a feature per lane (128 + 128 rows a CTA).  Returns the old value.
 extern "C" int rb_set_gemm_gated_stream(int v) { int old = g_tc_gated_stream; g_tc_gated_stream = v ? 1 : 0; return old; }
 
@@ -1837,9 +1837,12 @@ extern "C" int rb_gemm_bf16_swiglu(const void* X, const void* Wgu, void* act, in
         return launch_tc_persistent<128, 4, 1, 256>(mw, mx, act, T, F, K, ldc, 0, s, TcHeads{}, tc_rows(ex));
     }
     if (row_sumsq && T > 256) RB_REFUSE("gemm_swiglu: row factors over %d tokens need the persistent product", T);
-    // 65 .. 128 tokens: F / 64 CTAs, two to an SM.  (For 33 .. 64 tokens the same kernel, also with 64-token stages of
-    // 24 KB, is faster alone - 40 against 44 us at the 8B shape - but the decode step around it is not: 9.86 against
-    // 9.78 ms at batch 64; its 192 CTAs leave the product after it no SM to start on early.)
+    // 33 .. 128 tokens: F / 64 CTAs, two to an SM, nothing to reduce.  (The form with a feature per lane has one CTA to an SM from 33
+    // tokens on, in clusters: at the 4B shape 228 of them, 1.5 rounds.  Decode steps at 40 and 64 requests, context 140: 4B 3.10 -> 2.95
+    // and 3.55 -> 3.33 ms, 8B 3.93 -> 3.88 and 4.44 -> 4.33, eight layers of 32B 2.01 -> 1.93 and 2.14 -> 2.04; at 24 requests
+    // it is the slower one, 2.67 against 2.48 and 3.59 against 3.42 ms.)
+    if (T > 32 && T <= 64 && force_splits == 0 && g_tc_gated_stream)
+        return launch_tc_gated_stream<4, 64>(X, Wgu, act, T, F, K, ldx, ldw, ldc, ex, s);
     if (T > 64 && T <= 128 && force_splits == 0 && g_tc_gated_stream)
         return launch_tc_gated_stream<3, 128>(X, Wgu, act, T, F, K, ldx, ldw, ldc, ex, s);
     if (rb_tensor_map_bf16(X, T, K, ldx, bn, &mx)) return -1;
