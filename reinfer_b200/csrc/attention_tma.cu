@@ -73,6 +73,12 @@ struct FtShared {
     int abort_flag;
 };
 
+// 2^x by the special-function unit alone (what exp2f adds is for results below 2^-126, which are zero here); two units in the last place.
+__device__ __forceinline__ float ft_ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
 __device__ __forceinline__ void ft_ldsm_x4(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
@@ -149,7 +155,7 @@ __device__ __forceinline__ void ft_merge_weights(float* sF, float* sLse, int Gc,
 // KONLY: the pages hold keys only and the values are the keys themselves (latent attention without a rotated part): a key tile
 // is fetched once and used by both products, and a stage holds one tile.
 template <int HALVES, int NST, bool P5, bool KONLY>
-__global__ void __launch_bounds__(FT_THREADS, KONLY ? 2 : 1)      // (KONLY: two CTAs to an SM, by registers too)
+__global__ void __launch_bounds__(FT_THREADS, KONLY || HALVES <= 2 ? 2 : 1)      // (two CTAs to an SM, by registers too: three of their ten warps share a scheduler)
 fa_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const FtArgs a) {
     RB_TL(4);
     constexpr int D = HALVES * 64;
@@ -157,6 +163,9 @@ fa_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const FtArgs a)
     constexpr int STAGE = (KONLY ? 1 : 2) * KV_BYTES;
     static_assert(!(P5 && KONLY), "the 5-D map describes pages of keys and values");
     constexpr int Q_HALF = 16 * 128;
+    // Up to 128 dims a lane keeps its share of the query rows in registers for all tiles, loaded as the product wants them.
+    constexpr bool QREG = HALVES <= 2;
+    uint32_t qf[QREG ? D / 16 : 1][4];
     // byte offset of 16-byte chunk c of key `row` inside a key (or value) tile
     auto kv_off = [](int row, int c) -> uint32_t {
         return P5 ? (uint32_t)((row >> 3) * 2048 + (c >> 3) * 1024 + (row & 7) * 128 + (((c & 7) ^ (row & 7)) << 4))
@@ -177,10 +186,16 @@ fa_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const FtArgs a)
         sh->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // shared memory starts at zero: rows that no copy fills are then finite
-    for (int i = threadIdx.x; i < (NST * STAGE + HALVES * Q_HALF) / 16; i += FT_THREADS)
-        reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the zeroing precedes the TMA writes
+    // With a window a tile may hold pages that went back to the pool: no copy fills their rows, and they start at zero, so that they
+    // are finite.  (Rows beyond the request's length are set to zero in its last tile.)  100 KB of zeros take a CTA 0.8 us.
+    if (a.window > 0) {
+        for (int i = threadIdx.x; i < NST * STAGE / 16; i += FT_THREADS)
+            reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the zeroing precedes the TMA writes
+    }
+    if (!QREG)
+        for (int i = threadIdx.x; i < HALVES * Q_HALF / 16; i += FT_THREADS)
+            reinterpret_cast<uint4*>(sQ)[i] = make_uint4(0, 0, 0, 0);
     __syncthreads();
     if (threadIdx.x == 0) FT_T(1);
     pdl_trigger();
@@ -209,6 +224,18 @@ fa_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const FtArgs a)
         pdl_wait();
         RB_TL_MARK();
         if (threadIdx.x == 0) FT_T(2);
+        if (QREG) {
+            const bf16* q0 = a.q + ((size_t)tok * a.QH + head0 + (lane >> 2)) * a.d + 2 * (lane & 3);
+            const bool in0 = (lane >> 2) < a.Gc, in1 = (lane >> 2) + 8 < a.Gc;
+#pragma unroll
+            for (int ks = 0; ks < (QREG ? D / 16 : 1); ++ks)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const int c = ks * 16 + j * 8;                 // (d is a multiple of 8)
+                    qf[ks][2 * j] = in0 && c < a.d ? *reinterpret_cast<const uint32_t*>(q0 + c) : 0u;
+                    qf[ks][2 * j + 1] = in1 && c < a.d ? *reinterpret_cast<const uint32_t*>(q0 + (size_t)8 * a.d + c) : 0u;
+                }
+        } else {
         // Q rows (row r = query head head0 + r) into the swizzled layout, by the consumer warps that read them
         for (int i = threadIdx.x; i < a.Gc * (a.d / 8); i += FT_WARPS * 32) {
             const int row = i / (a.d / 8), c = i % (a.d / 8);
@@ -216,6 +243,7 @@ fa_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const FtArgs a)
             *reinterpret_cast<uint4*>(sQ + ft_off(row, c, Q_HALF)) = v;
         }
         asm volatile("bar.sync 1, %0;" ::"n"(FT_WARPS * 32) : "memory");
+        }
     }
 
     const int box_rows = min(a.page_size, FT_BN);
@@ -296,9 +324,10 @@ fa_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const FtArgs a)
                               gridDim.x * gridDim.y * gridDim.z);
     } else {
         // ---- consumer warps --------------------------------------------------------------------
+        bool landed = false;                                       // the next tile's barrier is looked at while this one is worked on
         for (int it = 0; it < n_tiles; ++it) {
             const int s = it % NST;
-            if (!mbar_wait(smem_u32(&sh->full[s]), (it / NST) & 1, abort_flag, 4)) break;
+            if (!landed && !mbar_wait(smem_u32(&sh->full[s]), (it / NST) & 1, abort_flag, 4)) break;
             if (it == 0 && threadIdx.x == 0) FT_T(3);
             const uint32_t sK = stages_u + s * STAGE, sV = KONLY ? sK : sK + KV_BYTES;
             const int k0 = (t_begin + it) * FT_BN;
@@ -320,12 +349,14 @@ fa_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const FtArgs a)
             for (int j = 0; j < 2; ++j) { sc[j][0] = sc[j][1] = sc[j][2] = sc[j][3] = 0.0f; }
 #pragma unroll
             for (int ks = 0; ks < D / 16; ++ks) {
-                uint32_t qa[4], kb[4];
-                ft_ldsm_x4(qa, sQ_u + ft_off((lane & 7) + 8 * ((lane >> 3) & 1), ks * 2 + (lane >> 4), Q_HALF));
+                uint32_t qs[4], kb[4];
+                if (!QREG) ft_ldsm_x4(qs, sQ_u + ft_off((lane & 7) + 8 * ((lane >> 3) & 1), ks * 2 + (lane >> 4), Q_HALF));
+                const uint32_t (&qa)[4] = QREG ? qf[QREG ? ks : 0] : qs;
                 ft_ldsm_x4(kb, sK + kv_off(koff + (lane & 7) + 8 * (lane >> 4), ks * 2 + ((lane >> 3) & 1)));
                 ft_mma(sc[0], qa, kb[0], kb[1]);
                 ft_mma(sc[1], qa, kb[2], kb[3]);
             }
+            landed = it + 1 < n_tiles && mbar_test(smem_u32(&sh->full[(it + 1) % NST]), ((it + 1) / NST) & 1);
             float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
@@ -352,18 +383,21 @@ fa_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const FtArgs a)
             mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
             const float mn0 = fmaxf(m[0], mx0), mn1 = fmaxf(m[1], mx1);
             const float b0 = mn0 == -INFINITY ? 0.0f : mn0, b1 = mn1 == -INFINITY ? 0.0f : mn1;
-            const float c0 = exp2f(m[0] - b0), c1 = exp2f(m[1] - b1);
+            const bool moved = mn0 != m[0] || mn1 != m[1];
+            const float c0 = ft_ex2(m[0] - b0), c1 = ft_ex2(m[1] - b1);
             m[0] = mn0; m[1] = mn1;
             uint32_t pa[4];
             {
-                const float e0 = exp2f(sc[0][0] - b0), e1 = exp2f(sc[0][1] - b0), e2 = exp2f(sc[0][2] - b1), e3 = exp2f(sc[0][3] - b1);
-                const float f0 = exp2f(sc[1][0] - b0), f1 = exp2f(sc[1][1] - b0), f2 = exp2f(sc[1][2] - b1), f3 = exp2f(sc[1][3] - b1);
+                const float e0 = ft_ex2(sc[0][0] - b0), e1 = ft_ex2(sc[0][1] - b0), e2 = ft_ex2(sc[0][2] - b1), e3 = ft_ex2(sc[0][3] - b1);
+                const float f0 = ft_ex2(sc[1][0] - b0), f1 = ft_ex2(sc[1][1] - b0), f2 = ft_ex2(sc[1][2] - b1), f3 = ft_ex2(sc[1][3] - b1);
                 l[0] = l[0] * c0 + (e0 + e1) + (f0 + f1);
                 l[1] = l[1] * c1 + (e2 + e3) + (f2 + f3);
                 pa[0] = ft_pack(e0, e1); pa[1] = ft_pack(e2, e3); pa[2] = ft_pack(f0, f1); pa[3] = ft_pack(f2, f3);
             }
+            if (__any_sync(0xffffffffu, moved)) {                  // (else both factors are 1 in every lane)
 #pragma unroll
-            for (int j = 0; j < D / 8; ++j) { o[j][0] *= c0; o[j][1] *= c0; o[j][2] *= c1; o[j][3] *= c1; }
+                for (int j = 0; j < D / 8; ++j) { o[j][0] *= c0; o[j][1] *= c0; o[j][2] *= c1; o[j][3] *= c1; }
+            }
 #pragma unroll
             for (int dp = 0; dp < D / 16; ++dp) {
                 uint32_t vb[4];
