@@ -198,7 +198,6 @@ fa_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const FtArgs a)
             reinterpret_cast<uint4*>(sQ)[i] = make_uint4(0, 0, 0, 0);
     __syncthreads();
     if (threadIdx.x == 0) FT_T(1);
-    pdl_trigger();
 
     // The step's tables (lengths, block table) were complete before its first kernel began, and the keys of
     // earlier positions were written by earlier steps: both may be read while the kernels before this one still
@@ -222,6 +221,9 @@ fa_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const FtArgs a)
 
     if (warp < FT_WARPS) {
         pdl_wait();
+        // The product after this kernel may fetch its weights while the attention waits for keys and reduces, not before: it would take
+        // the memory's time from the product in front, which this kernel waits for.
+        pdl_trigger();
         RB_TL_MARK();
         if (threadIdx.x == 0) FT_T(2);
         if (QREG) {

@@ -200,7 +200,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     if (warp == 0) {
         // Weights never change, so their first tiles are fetched at once, while the kernels
         // before this one may still be running; the activations wait for them to finish.
-        pdl_trigger();
         const int pre = min(nkb, STAGES);
         for (int kb = 0; kb < pre; ++kb) {
             const uint32_t full = smem_u32(&sh->full[kb]);
@@ -238,6 +237,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 if (!ok) break;
             }
             if (kb == 0 && lead) TL(2);
+            // The kernel after this one may begin, and fetch its weights, when this one has little left to fetch.  (When it may begin at once,
+            // what it fetches delays this kernel's own weights, and memory idles later, while this one reduces and stores.  Decode
+            // steps: 4B at 64 and 16 requests 3.33 -> 3.20 and 2.60 -> 2.54 ms, 8B at eight 3.25 -> 3.20, eight layers of 32B at six
+            // 1.68 -> 1.65; the recurrent design at eight 0.497 -> 0.480, the mixture 0.797 -> 0.770.)  A long share of K says so when
+            // its last loads are on their way, a short one, all of whose loads go out at once, when three blocks are left: the other
+            // way round the 8B shape loses 0.5 % at one request, the recurrent design 1 % at eight.
+            if (kb == max(0, nkb - (nkb >= 10 ? STAGES : 3))) pdl_trigger();
             const uint32_t a = smem_base + s * STAGE_BYTES;
             const uint64_t da = make_smem_desc(a), db = make_smem_desc(a + W_BYTES);
             const uint64_t da2 = make_smem_desc(a + W1_BYTES);
@@ -1144,7 +1150,6 @@ gemm_tc_gated_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __g
     int issued = 0;
 
     if (warp == 0) {
-        pdl_trigger();
         const int pre = min(nkb, STAGES);
         for (int kb = 0; kb < pre; ++kb) {                         // the weights never change: fetched at once
             const uint32_t full = full0 + 8 * kb;
@@ -1167,7 +1172,9 @@ gemm_tc_gated_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __g
             tma_load_2d_lead(dst + W_BYTES, &map_x, kb * TC_BK, 0, full, lead);
             issued = kb + 1;
         }
-        // this CTA's weights are on their way: the weights that the next product streams are called into L2
+        // this CTA's weights are on their way: the kernel after this one may begin (not before, see gemm_tc_kernel), and the weights that
+        // the next product streams are called into L2
+        pdl_trigger();
         if (lead) l2_prefetch_share(ex.next_w, ex.next_bytes, blockIdx.x, gridDim.x);
     } else if (warp == 1) {
         constexpr uint32_t idesc = make_idesc(2 * TCS_ROWS);
