@@ -265,27 +265,41 @@ add_rmsnorm_cluster_kernel(float* __restrict__ x, const float* __restrict__ delt
 // a thread in flight before the first is used.  (The 32-bit path keeps the scalar kernel above, whose sums do not
 // depend on how many rows a step brings.)
 constexpr int RV_THREADS = 256;
-template <typename TW, int VPER>
-__global__ void __launch_bounds__(RV_THREADS)
+__device__ __forceinline__ float4 rv_weights(const float* w) { return make_float4(w[0], w[1], w[2], w[3]); }
+__device__ __forceinline__ float4 rv_weights(const bf16* w) {
+    const uint2 p = *reinterpret_cast<const uint2*>(w);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&p.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&p.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+template <typename TW, int VPER, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 add_rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ delta, int n_delta, long long delta_stride,
                        const TW* __restrict__ w, bf16* __restrict__ out, int h, float eps) {
     RB_TL(2);
     __shared__ float red[32];
-    pdl_trigger(); pdl_wait();
+    pdl_trigger();
+    // the norm's weights never change: they are fetched while the kernels before this one still run
+    float4 wv[VPER];
+#pragma unroll
+    for (int k = 0; k < VPER; ++k) {
+        const int i = (threadIdx.x + k * THREADS) * 4;
+        wv[k] = i < h ? rv_weights(w + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    pdl_wait();
     RB_TL_MARK();
     const size_t row = (size_t)blockIdx.x * h;
     float4 v[VPER];
     float ss = 0.0f;
 #pragma unroll
     for (int k = 0; k < VPER; ++k) {
-        const int i = (threadIdx.x + k * RV_THREADS) * 4;
+        const int i = (threadIdx.x + k * THREADS) * 4;
         v[k] = i < h ? *reinterpret_cast<const float4*>(x + row + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (delta) {
         for (int p = 0; p < n_delta; ++p) {                        // ascending: a fixed order
 #pragma unroll
             for (int k = 0; k < VPER; ++k) {
-                const int i = (threadIdx.x + k * RV_THREADS) * 4;
+                const int i = (threadIdx.x + k * THREADS) * 4;
                 if (i < h) {
                     const float4 d = *reinterpret_cast<const float4*>(delta + (size_t)p * delta_stride + row + i);
                     v[k].x += d.x; v[k].y += d.y; v[k].z += d.z; v[k].w += d.w;
@@ -294,7 +308,7 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ delta, i
         }
 #pragma unroll
         for (int k = 0; k < VPER; ++k) {
-            const int i = (threadIdx.x + k * RV_THREADS) * 4;
+            const int i = (threadIdx.x + k * THREADS) * 4;
             if (i < h) *reinterpret_cast<float4*>(x + row + i) = v[k];
         }
     }
@@ -304,24 +318,29 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ delta, i
     const float rstd = 1.0f / sqrtf(total / (float)h + eps);
 #pragma unroll
     for (int k = 0; k < VPER; ++k) {
-        const int i = (threadIdx.x + k * RV_THREADS) * 4;
+        const int i = (threadIdx.x + k * THREADS) * 4;
         if (i < h) {
-            const __nv_bfloat162 lo = __floats2bfloat162_rn(v[k].x * rstd * to_f32(w[i]), v[k].y * rstd * to_f32(w[i + 1]));
-            const __nv_bfloat162 hi = __floats2bfloat162_rn(v[k].z * rstd * to_f32(w[i + 2]), v[k].w * rstd * to_f32(w[i + 3]));
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(v[k].x * rstd * wv[k].x, v[k].y * rstd * wv[k].y);
+            const __nv_bfloat162 hi = __floats2bfloat162_rn(v[k].z * rstd * wv[k].z, v[k].w * rstd * wv[k].w);
             uint2 pk;
             pk.x = *reinterpret_cast<const uint32_t*>(&lo); pk.y = *reinterpret_cast<const uint32_t*>(&hi);
             *reinterpret_cast<uint2*>(out + row + i) = pk;
         }
     }
 }
+// Few enough threads a row that its loads are most of what a thread does, and no more of them than the row has pieces: 2,048 rows, their
+// data out of L2, by width 2,048 / 2,560 / 4,096 / 5,120: 6.5 / 7.4 / 11.7 / 14.7 us with 128 threads, 7.7 / 8.5 / 11.0 / 13.5 with
+// 256, 12.7 / 13.6 / 15.6 / 17.4 with 512 (256, the weights read behind the sum, in 2, 4, 4 and 8 pieces: 8.4 / 10.0 / 12.7 / 16.9).
 template <typename TW>
 static int launch_add_rmsnorm_vec(float* x, const float* delta, int n_delta, long long delta_stride, const TW* w, bf16* out,
                                   int rows, int h, float eps, cudaStream_t s) {
-    const int vper = rb_ceil_div(h, RV_THREADS * 4);
-    if (vper <= 1) return rb_launch(add_rmsnorm_vec_kernel<TW, 1>, dim3(rows), dim3(RV_THREADS), 0, s, x, delta, n_delta, delta_stride, w, out, h, eps);
-    if (vper <= 2) return rb_launch(add_rmsnorm_vec_kernel<TW, 2>, dim3(rows), dim3(RV_THREADS), 0, s, x, delta, n_delta, delta_stride, w, out, h, eps);
-    if (vper <= 4) return rb_launch(add_rmsnorm_vec_kernel<TW, 4>, dim3(rows), dim3(RV_THREADS), 0, s, x, delta, n_delta, delta_stride, w, out, h, eps);
-    return rb_launch(add_rmsnorm_vec_kernel<TW, 8>, dim3(rows), dim3(RV_THREADS), 0, s, x, delta, n_delta, delta_stride, w, out, h, eps);
+    const int threads = h <= 128 * 4 * 5 ? 128 : RV_THREADS, pieces = rb_ceil_div(h, threads * 4);
+#define RB_RV(V, T) if (threads == T && pieces <= V) \
+        return rb_launch(add_rmsnorm_vec_kernel<TW, V, T>, dim3(rows), dim3(T), 0, s, x, delta, n_delta, delta_stride, w, out, h, eps)
+    RB_RV(1, 128); RB_RV(2, 128); RB_RV(3, 128); RB_RV(4, 128); RB_RV(5, 128);
+    RB_RV(3, 256); RB_RV(4, 256); RB_RV(5, 256); RB_RV(6, 256); RB_RV(8, 256);
+#undef RB_RV
+    RB_REFUSE("rmsnorm: a row of %d", h);
 }
 
 // An RMS norm whose division is left to the product that reads it:  x[r,:] += sum_p delta[p][r,:] (ascending),
@@ -423,7 +442,7 @@ extern "C" int rb_add_rmsnorm(float* x, const void* delta, int delta_dtype, int 
                                      (const float*)delta, n_delta, delta_stride, (const bf16*)w, (bf16*)out, row_idx, h, eps);
     }
     if (out_dtype == RB_BF16 && dd == RB_F32 && !row_idx && rows > 64 && h % 4 == 0 && h <= RV_THREADS * 4 * 8 &&
-        ((((uintptr_t)x | (uintptr_t)delta) & 15) == 0) && (((uintptr_t)out) & 7) == 0 && (!delta || delta_stride % 4 == 0)) {
+        ((((uintptr_t)x | (uintptr_t)delta) & 15) == 0) && (((uintptr_t)out | (w_dtype == RB_BF16 ? (uintptr_t)w : 0)) & 7) == 0 && (!delta || delta_stride % 4 == 0)) {
         if (w_dtype == RB_F32) return launch_add_rmsnorm_vec<float>(x, (const float*)delta, n_delta, delta_stride, (const float*)w, (bf16*)out, rows, h, eps, s);
         if (w_dtype == RB_BF16) return launch_add_rmsnorm_vec<bf16>(x, (const float*)delta, n_delta, delta_stride, (const bf16*)w, (bf16*)out, rows, h, eps, s);
     }
