@@ -30,12 +30,76 @@ __global__ void dyt_kernel(float* __restrict__ x, const float* __restrict__ delt
     }
 }
 
+// The same for bfloat16 rows of whole 16-byte pieces: float4 loads, all on their way before the first is used, weights ahead of the wait.
+// 2,048 rows of 2,048
+// between two products: 6.2 us, 11.0 by elements.
+#define DV_THREADS 128
+template <int VPER>
+__global__ void __launch_bounds__(DV_THREADS)
+dyt_vec_kernel(float* __restrict__ x, const float* __restrict__ delta, int n_delta, long long delta_stride, const bf16* __restrict__ w,
+               const bf16* __restrict__ b, const bf16* __restrict__ alpha, bf16* __restrict__ out, const int* __restrict__ row_idx, int h) {
+    pdl_trigger();
+    const float a = to_f32(alpha[0]);
+    uint2 wv[VPER], bv[VPER];
+#pragma unroll
+    for (int k = 0; k < VPER; ++k) {
+        const int i = (threadIdx.x + k * DV_THREADS) * 4;
+        wv[k] = bv[k] = make_uint2(0, 0);
+        if (i < h) { wv[k] = *reinterpret_cast<const uint2*>(w + i); bv[k] = *reinterpret_cast<const uint2*>(b + i); }
+    }
+    pdl_wait();
+    const int r = blockIdx.x;
+    float* xr = x + (row_idx ? (size_t)row_idx[r] : (size_t)r) * h;
+    float4 v[VPER];
+#pragma unroll
+    for (int k = 0; k < VPER; ++k) {
+        const int i = (threadIdx.x + k * DV_THREADS) * 4;
+        v[k] = i < h ? *reinterpret_cast<const float4*>(xr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (delta) {
+        const float* dr = delta + (row_idx ? (size_t)row_idx[r] : (size_t)r) * h;
+        for (int p = 0; p < n_delta; ++p)                              // ascending
+#pragma unroll
+            for (int k = 0; k < VPER; ++k) {
+                const int i = (threadIdx.x + k * DV_THREADS) * 4;
+                if (i < h) {
+                    const float4 d = *reinterpret_cast<const float4*>(dr + (size_t)p * delta_stride + i);
+                    v[k].x += d.x; v[k].y += d.y; v[k].z += d.z; v[k].w += d.w;
+                }
+            }
+        if (!row_idx)
+#pragma unroll
+            for (int k = 0; k < VPER; ++k) {
+                const int i = (threadIdx.x + k * DV_THREADS) * 4;
+                if (i < h) *reinterpret_cast<float4*>(xr + i) = v[k];
+            }
+    }
+#pragma unroll
+    for (int k = 0; k < VPER; ++k) {
+        const int i = (threadIdx.x + k * DV_THREADS) * 4;
+        if (i >= h) continue;
+        const float2 w0 = __bfloat1622float2(*(const __nv_bfloat162*)&wv[k].x), w1 = __bfloat1622float2(*(const __nv_bfloat162*)&wv[k].y);
+        const float2 b0 = __bfloat1622float2(*(const __nv_bfloat162*)&bv[k].x), b1 = __bfloat1622float2(*(const __nv_bfloat162*)&bv[k].y);
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(fmaf(tanhf(a * v[k].x), w0.x, b0.x), fmaf(tanhf(a * v[k].y), w0.y, b0.y));
+        const __nv_bfloat162 hi = __floats2bfloat162_rn(fmaf(tanhf(a * v[k].z), w1.x, b1.x), fmaf(tanhf(a * v[k].w), w1.y, b1.y));
+        *reinterpret_cast<uint2*>(out + (size_t)r * h + i) = make_uint2(*(const uint32_t*)&lo, *(const uint32_t*)&hi);
+    }
+}
+
 extern "C" int rb_dyt(float* x, const float* delta, int n_delta, long long delta_stride, const void* w, const void* b,
                       const void* alpha, int w_dtype, void* out, int out_dtype, const int* row_idx, int rows, int h,
                       void* stream) {
     if (rows <= 0) return 0;
     if (h <= 0) RB_REFUSE("dyt: width %d", h);
     cudaStream_t s = (cudaStream_t)stream;
+    if (w_dtype == RB_BF16 && out_dtype == RB_BF16 && h % 4 == 0 && h <= DV_THREADS * 4 * 8 && delta_stride % 4 == 0 &&
+        (((uintptr_t)x | (uintptr_t)delta) & 15) == 0 && (((uintptr_t)w | (uintptr_t)b | (uintptr_t)out) & 7) == 0) {
+        const int pieces = rb_ceil_div(h, DV_THREADS * 4);
+#define RB_DV(V) if (pieces <= V) return rb_launch(dyt_vec_kernel<V>, dim3(rows), dim3(DV_THREADS), 0, s, x, delta, n_delta, delta_stride, \
+                                                   (const bf16*)w, (const bf16*)b, (const bf16*)alpha, (bf16*)out, row_idx, h)
+        RB_DV(1); RB_DV(2); RB_DV(4); RB_DV(5); RB_DV(8);
+#undef RB_DV
+    }
     const int threads = h >= 2048 ? 512 : (h >= 512 ? 256 : 128);
 #define RB_DYT(TW, TO) return rb_launch(dyt_kernel<TW, TO>, dim3(rows), dim3(threads), 0, s, x, delta, n_delta, delta_stride, \
                                         (const TW*)w, (const TW*)b, (const TW*)alpha, (TO*)out, row_idx, h)
@@ -110,6 +174,52 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o, const float* 
         dst[i] = from_f32<TA>(src[i] * rstd * wv[i] * gv * out_scale);
     }
 }
+// The same for bfloat16 heads of 64, 128 or 256: LANES lanes a head with PER pieces of four neighbours each, every load on its way before
+// the head's sum is formed, the weight ahead of the wait.  2,048 tokens, 32 heads of 64 / 16 of 128:
+// 10.3 / 10.1 us, 27.5 / 17.5 element by element.
+template <int LANES, int PER>
+__global__ void __launch_bounds__(128)
+head_norm_gate_vec_kernel(const float* __restrict__ o, const float* __restrict__ w, int w_heads, const bf16* __restrict__ gate, long long ldg, int act,
+                          bf16* __restrict__ out, long long ldo, int n_tokens, int H, float eps, float out_scale) {
+    constexpr int DV = LANES * PER * 4;
+    pdl_trigger();
+    const long long hd = ((long long)blockIdx.x * 128 + threadIdx.x) / LANES;
+    const int l = threadIdx.x % LANES;
+    const bool live = hd < (long long)n_tokens * H;
+    const int t = live ? (int)(hd / H) : 0, hh = live ? (int)(hd % H) : 0;
+    float4 wv[PER], v[PER];
+    uint2 g[PER];
+#pragma unroll
+    for (int k = 0; k < PER; ++k) wv[k] = *reinterpret_cast<const float4*>(w + (w_heads ? (size_t)hh * DV : 0) + (k * LANES + l) * 4);
+    pdl_wait();
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int i = (k * LANES + l) * 4;
+        v[k] = *reinterpret_cast<const float4*>(o + ((size_t)t * H + hh) * DV + i);
+        g[k] = *reinterpret_cast<const uint2*>(gate + (size_t)t * ldg + (size_t)hh * DV + i);
+    }
+    float ss = 0.0f;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) ss += (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
+#pragma unroll
+    for (int s = LANES / 2; s > 0; s >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, s);
+    const float rstd = 1.0f / sqrtf(ss / (float)DV + eps);
+    if (!live) return;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const float2 g0 = __bfloat1622float2(*(const __nv_bfloat162*)&g[k].x), g1 = __bfloat1622float2(*(const __nv_bfloat162*)&g[k].y);
+        const float z[4] = {g0.x, g0.y, g1.x, g1.y}, a[4] = {v[k].x, v[k].y, v[k].z, v[k].w}, b[4] = {wv[k].x, wv[k].y, wv[k].z, wv[k].w};
+        float r[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float sg = 1.0f / (1.0f + expf(-z[j]));
+            r[j] = a[j] * rstd * b[j] * (act == 1 ? z[j] * sg : sg) * out_scale;
+        }
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(r[0], r[1]), hi = __floats2bfloat162_rn(r[2], r[3]);
+        *reinterpret_cast<uint2*>(out + (size_t)t * ldo + (size_t)hh * DV + (k * LANES + l) * 4) = make_uint2(*(const uint32_t*)&lo, *(const uint32_t*)&hi);
+    }
+}
+
 extern "C" int rb_head_norm_gate(const float* o, const float* w, int w_heads, const void* gate, long long ldg, int act,
                                  void* out, long long ldo, int dtype, int n_tokens, int H, int dv, float eps, float out_scale,
                                  void* stream) {
@@ -118,6 +228,15 @@ extern "C" int rb_head_norm_gate(const float* o, const float* w, int w_heads, co
     if (act != 0 && act != 1) RB_REFUSE("head_norm_gate: gate function %d", act);
     const int blocks = rb_ceil_div((long long)n_tokens * H, 4);
     cudaStream_t s = (cudaStream_t)stream;
+    if (dtype == RB_BF16 && (dv == 64 || dv == 128 || dv == 256) && ldg % 4 == 0 && ldo % 4 == 0 && (((uintptr_t)o | (uintptr_t)w) & 15) == 0 &&
+        (((uintptr_t)gate | (uintptr_t)out) & 7) == 0) {
+#define RB_HV(L, P) return rb_launch(head_norm_gate_vec_kernel<L, P>, dim3(rb_ceil_div((long long)n_tokens * H * L, 128)), dim3(128), 0, s, o, w, w_heads, \
+                                     (const bf16*)gate, ldg, act, (bf16*)out, ldo, n_tokens, H, eps, out_scale)
+        if (dv == 64) RB_HV(16, 1);
+        if (dv == 128) RB_HV(32, 1);
+        RB_HV(32, 2);
+#undef RB_HV
+    }
     if (dtype == RB_F32) return rb_launch(head_norm_gate_kernel<float>, dim3(blocks), dim3(128), 0, s, o, w, w_heads, (const float*)gate, ldg, act, (float*)out, ldo, n_tokens, H, dv, eps, out_scale);
     if (dtype == RB_BF16) return rb_launch(head_norm_gate_kernel<bf16>, dim3(blocks), dim3(128), 0, s, o, w, w_heads, (const bf16*)gate, ldg, act, (bf16*)out, ldo, n_tokens, H, dv, eps, out_scale);
     RB_REFUSE("head_norm_gate: dtype %d", dtype);

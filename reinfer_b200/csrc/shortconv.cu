@@ -11,6 +11,7 @@
 #define RC_MAX_TAPS 8
 #define RC_SEG 64
 #define RC_THREADS 128
+#define RC_AHEAD 8                            // inputs that a thread has asked for ahead of their use
 
 template <typename TA>
 __global__ void __launch_bounds__(RC_THREADS)
@@ -42,8 +43,20 @@ shortconv_kernel(const TA* __restrict__ u, long long ldu, const float* __restric
         }
     }
     const int end = min(a + RC_SEG, n);
-    for (int i = a; i < end; ++i) {
-        const float cur = to_f32(u[(size_t)(s0 + i) * ldu + c]);
+    // Eight inputs ahead: the segment is one chain of loads otherwise (2,048 tokens of three requests, 3,072 channels: 30 us,
+    // 22 like this).
+    TA next[RC_AHEAD];
+#pragma unroll
+    for (int q = 0; q < RC_AHEAD; ++q) next[q] = u[(size_t)(s0 + min(a + q, end - 1)) * ldu + c];
+    for (int i0 = a; i0 < end; i0 += RC_AHEAD) {
+        TA now[RC_AHEAD];
+#pragma unroll
+        for (int q = 0; q < RC_AHEAD; ++q) { now[q] = next[q]; next[q] = u[(size_t)(s0 + min(i0 + RC_AHEAD + q, end - 1)) * ldu + c]; }
+#pragma unroll
+        for (int q = 0; q < RC_AHEAD; ++q) {
+        const int i = i0 + q;
+        if (i >= end) break;
+        const float cur = to_f32(now[q]);
         float acc = 0.0f;
 #pragma unroll
         for (int j = 0; j < RC_MAX_TAPS - 1; ++j) acc = fmaf(wv[j], win[j], acc);
@@ -53,6 +66,7 @@ shortconv_kernel(const TA* __restrict__ u, long long ldu, const float* __restric
 #pragma unroll
         for (int j = 0; j < RC_MAX_TAPS - 2; ++j) win[j] = win[j + 1];
         win[RC_MAX_TAPS - 2] = cur;
+        }
     }
     if (update) {
 #pragma unroll
@@ -151,12 +165,40 @@ __global__ void unit_heads_append_kernel(const TA* __restrict__ x, long long ldx
         for (int i = lane; i < dk; i += 32) dst[i] = from_f32<TC>(to_f32(src[i]) * rstd);
     }
 }
+// The same for bfloat16 heads of 128: four neighbours a lane.  520 tokens, 16 + 4 + 4 heads: 3.8 us, 5.2 element by element.
+__global__ void __launch_bounds__(128)
+unit_heads_append_128_kernel(const bf16* __restrict__ x, long long ldx, const int* __restrict__ kv_slot, bf16* __restrict__ q_out,
+                             bf16* __restrict__ cache, int n_tokens, int QH, int KH, int page_size, float eps) {
+    pdl_trigger(); pdl_wait();
+    const int heads = QH + 2 * KH, lane = threadIdx.x & 31;
+    const long long wg = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (wg >= (long long)n_tokens * heads) return;
+    const int t = (int)(wg / heads), hh = (int)(wg % heads);
+    uint2 p = *reinterpret_cast<const uint2*>(x + (size_t)t * ldx + (size_t)hh * 128 + lane * 4);
+    const int slot = kv_slot ? kv_slot[t] : -1;
+    if (hh >= QH && slot < 0) return;
+    if (hh < QH + KH) {
+        const float2 a = __bfloat1622float2(*(const __nv_bfloat162*)&p.x), b = __bfloat1622float2(*(const __nv_bfloat162*)&p.y);
+        const float rstd = 1.0f / sqrtf(warp_sum((a.x * a.x + a.y * a.y) + (b.x * b.x + b.y * b.y)) / 128.0f + eps);
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(a.x * rstd, a.y * rstd), hi = __floats2bfloat162_rn(b.x * rstd, b.y * rstd);
+        p = make_uint2(*(const uint32_t*)&lo, *(const uint32_t*)&hi);
+    }
+    bf16* dst = q_out + ((size_t)t * QH + hh) * 128;
+    if (hh >= QH) {                                        // a page: keys [KH][page_size][128], then values
+        const int kh = hh < QH + KH ? hh - QH : hh - QH - KH;
+        dst = cache + (size_t)(slot / page_size) * KH * page_size * 256 + (hh < QH + KH ? 0 : (size_t)KH * page_size * 128) +
+              ((size_t)kh * page_size + slot % page_size) * 128;
+    }
+    *reinterpret_cast<uint2*>(dst + lane * 4) = p;
+}
 extern "C" int rb_unit_heads_append(const void* x, long long ldx, const int* kv_slot, void* q_out, void* cache, int dtype,
                                     int n_tokens, int QH, int KH, int dk, int dv, int page_size, float eps, void* stream) {
     if (n_tokens <= 0) return 0;
     if (QH <= 0 || KH <= 0 || dk <= 0 || dv <= 0 || page_size <= 0) RB_REFUSE("unit_heads_append: heads %d/%d sizes %d/%d page %d", QH, KH, dk, dv, page_size);
     const int blocks = rb_ceil_div((long long)n_tokens * (QH + 2 * KH), 4);
     cudaStream_t s = (cudaStream_t)stream;
+    if (dtype == RB_BF16 && dk == 128 && dv == 128 && ldx % 4 == 0 && (((uintptr_t)x | (uintptr_t)q_out | (uintptr_t)cache) & 7) == 0)
+        return rb_launch(unit_heads_append_128_kernel, dim3(blocks), dim3(128), 0, s, (const bf16*)x, ldx, kv_slot, (bf16*)q_out, (bf16*)cache, n_tokens, QH, KH, page_size, eps);
     if (dtype == RB_F32) return rb_launch(unit_heads_append_kernel<float, float>, dim3(blocks), dim3(128), 0, s, (const float*)x, ldx, kv_slot, (float*)q_out, (float*)cache, n_tokens, QH, KH, dk, dv, page_size, eps);
     if (dtype == RB_BF16) return rb_launch(unit_heads_append_kernel<bf16, bf16>, dim3(blocks), dim3(128), 0, s, (const bf16*)x, ldx, kv_slot, (bf16*)q_out, (bf16*)cache, n_tokens, QH, KH, dk, dv, page_size, eps);
     RB_REFUSE("unit_heads_append: dtype %d", dtype);
