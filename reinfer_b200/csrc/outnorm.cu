@@ -3,7 +3,8 @@
 // y comes as one float row or as a stack of partial sums that a split product left (added in ascending order);
 // x is the float residual stream and is updated in place.  Optionally the new x is also written rounded to
 // bfloat16: the next sublayer's products read the stream itself, not a norm of it.  One CTA per row; the row of
-// y lives in shared memory between the two passes.  The order of every sum depends on the width alone.
+// y lives in registers between the two passes (wider than 4,096, or not in 16-byte pieces: in shared memory).  The order of every
+// sum depends on the width and on whether y is a stack.
 // The kernel can also leave the rows of what reads the stream next: of one RMS norm without its division (next_rows and
 // the row's sum of squares), or complete rows of one or two RMS norms (RbNext: bfloat16 or float) - two where mixer and
 // feed-forward of the next layer each have a norm of their own over the same stream.  rb_rmsnorm_pair makes those
@@ -195,6 +196,105 @@ __global__ void residual_outnorm_kernel(float* __restrict__ x, const float* __re
     }
 }
 
+// The same for a row that is at most VPER float4 a thread: everything stays in registers, the weights are there before the kernels in
+// front are done, and the stream's row is asked for together with the sums, not behind their total.  A stack of partial sums is
+// many loads and few rows: one float4 a thread, so that all are in flight (8 rows of 2,048, 14 sums: 5.2 -> 3.6 us, the step of
+// the mixture's eight chats 26 -> 24 ms).  One row of y per row of x is as many float4 as keep a CTA at 256 threads (2,048 rows of
+// 2,048: 14.2 -> 12.9 us, 6.2 TB/s, 512 threads with one each 17.0; of 4,096: 28.0 -> 24.5; 8 rows of 2,048: 3.2 -> 2.6).
+template <typename TW, int VPER, int THREADS>
+__global__ void __launch_bounds__(THREADS)
+residual_outnorm_regs_kernel(float* __restrict__ x, const float* __restrict__ y, int n_parts, long long part_stride, const TW* __restrict__ w,
+                             bf16* __restrict__ rounded, int h, float eps, float mult, const float* __restrict__ extra_a,
+                             const void* __restrict__ extra_src, int extra_bf16, const float* __restrict__ next_w, bf16* __restrict__ next_rows,
+                             float* __restrict__ next_sumsq, int next_parts, RbNext nx) {
+    __shared__ float red[32];
+    pdl_trigger();
+    const int r = blockIdx.x, step = blockDim.x * 4;
+    const size_t row0 = (size_t)r * h;
+    float wv[VPER][4] = {}, nw[VPER][4] = {};
+#pragma unroll
+    for (int j = 0; j < VPER; ++j) {
+        const int i = threadIdx.x * 4 + j * step;
+        if (i < h) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                wv[j][k] = to_f32(w[i + k]);
+                if (next_rows) nw[j][k] = next_w[i + k];
+            }
+        }
+    }
+    pdl_wait();
+    const float ea = extra_a ? extra_a[r] : 0.0f;
+    float4 o[VPER], v[VPER];
+    float ss = 0.0f;
+#pragma unroll
+    for (int j = 0; j < VPER; ++j) {
+        const int i = threadIdx.x * 4 + j * step;
+        o[j] = v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < h) {
+            o[j] = *reinterpret_cast<const float4*>(x + row0 + i);
+            v[j] = *reinterpret_cast<const float4*>(y + row0 + i);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < VPER; ++j) {
+        const int i = threadIdx.x * 4 + j * step;
+        float4& a = v[j];
+        if (i < h) {
+            for (int s0 = 1; s0 < n_parts; s0 += 8) {          // eight partial sums in flight, added in ascending order
+                float4 d[8];
+#pragma unroll
+                for (int p = 0; p < 8; ++p)
+                    d[p] = s0 + p < n_parts ? *reinterpret_cast<const float4*>(y + row0 + i + (size_t)(s0 + p) * part_stride)
+                                            : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int p = 0; p < 8; ++p) if (s0 + p < n_parts) { a.x += d[p].x; a.y += d[p].y; a.z += d[p].z; a.w += d[p].w; }
+            }
+            if (extra_a) {
+                float e[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    e[k] = extra_bf16 ? to_f32(((const bf16*)extra_src)[row0 + i + k]) : ((const float*)extra_src)[row0 + i + k];
+                a.x = fmaf(ea, e[0], a.x); a.y = fmaf(ea, e[1], a.y); a.z = fmaf(ea, e[2], a.z); a.w = fmaf(ea, e[3], a.w);
+            }
+        }
+        ss += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
+    }
+    const float f = mult / sqrtf(block_sum(ss, red) / (float)h + eps);
+    const auto pack = [](float a, float b, float c, float d) {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, d);
+        return make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    };
+    float ss2 = 0.0f;
+#pragma unroll
+    for (int j = 0; j < VPER; ++j) {
+        const int i = threadIdx.x * 4 + j * step;
+        o[j].x += v[j].x * f * wv[j][0]; o[j].y += v[j].y * f * wv[j][1]; o[j].z += v[j].z * f * wv[j][2]; o[j].w += v[j].w * f * wv[j][3];
+        ss2 += o[j].x * o[j].x + o[j].y * o[j].y + o[j].z * o[j].z + o[j].w * o[j].w;
+        if (i < h) {
+            *reinterpret_cast<float4*>(x + row0 + i) = o[j];
+            if (rounded) *reinterpret_cast<uint2*>(rounded + row0 + i) = pack(o[j].x, o[j].y, o[j].z, o[j].w);
+            if (next_rows) *reinterpret_cast<uint2*>(next_rows + row0 + i) = pack(o[j].x * nw[j][0], o[j].y * nw[j][1], o[j].z * nw[j][2], o[j].w * nw[j][3]);
+        }
+    }
+    if (!next_rows && !nx.w1) return;
+    const float total = block_sum(ss2, red);
+    if (next_rows) {                                           // (the reader adds a row's parts: the whole sum is the first, the others are zero)
+        for (int p = threadIdx.x; p < next_parts; p += blockDim.x) next_sumsq[(size_t)r * next_parts + p] = p == 0 ? total : 0.0f;
+        return;
+    }
+    const float rstd = 1.0f / sqrtf(total / (float)h + nx.eps);
+#pragma unroll
+    for (int j = 0; j < VPER; ++j) {
+        const int i = threadIdx.x * 4 + j * step;
+        if (i < h) {
+            const float ov[4] = {o[j].x, o[j].y, o[j].z, o[j].w};
+            next_store<4>(nx, nx.w1, nx.rows1, row0, i, ov, rstd);
+            if (nx.w2) next_store<4>(nx, nx.w2, nx.rows2, row0, i, ov, rstd);
+        }
+    }
+}
+
 // y: n_parts stacked [rows, h] float arrays, part_stride elements apart.  rounded: bfloat16 [rows, h] or null.
 // extra_a [rows] float with extra_src [rows, h] (float or bfloat16), or neither.  next_w [h] float with next_rows
 // [rows, h] bfloat16 and next_sumsq [rows, next_parts] float, or none of them: the rows of the norm that reads the
@@ -218,11 +318,22 @@ extern "C" int rb_residual_outnorm(float* x, const float* y, int n_parts, long l
     if (smem > 200 * 1024) RB_REFUSE("outnorm: a row of %d floats does not fit shared memory", h);
     cudaStream_t s = (cudaStream_t)stream;
     const bool vec = h % 4 == 0 && part_stride % 4 == 0 && ((uintptr_t)x | (uintptr_t)y) % 16 == 0 && (!rounded || (uintptr_t)rounded % 8 == 0);
-    // a stack of partial sums over few rows: a thread per 16 bytes of the row, so that all of a row's loads are in flight
-    // at once (the order of the sums is then a function of the width and of whether the input is a stack - never of
-    // the other rows)
+    // (the order of the sums is a function of the width and of whether the input is a stack - never of the other rows, nor of what
+    // the kernel leaves besides the stream)
+    if (vec && h <= 4096) {
+        const int per = n_parts > 1 || h <= 1024 ? 1 : (h <= 2048 ? 2 : 4), threads = rb_ceil_div(h / 4, 32 * per) * 32;
+#define RB_ONR(TW, VPER, THREADS) return rb_launch(residual_outnorm_regs_kernel<TW, VPER, THREADS>, dim3(rows), dim3(threads), 0, s, x, y, n_parts, \
+        part_stride, (const TW*)w, (bf16*)rounded, h, eps, mult, extra_a, extra_src, extra_dtype == RB_BF16 ? 1 : 0, \
+        next_w, (bf16*)next_rows, next_sumsq, next_parts, nx)
+#define RB_ONW(TW) do { if (per == 4) RB_ONR(TW, 4, 256); if (per == 2) RB_ONR(TW, 2, 256); if (threads <= 256) RB_ONR(TW, 1, 256); RB_ONR(TW, 1, 1024); } while (0)
+        if (w_dtype == RB_F32) RB_ONW(float);
+        if (w_dtype == RB_BF16) RB_ONW(bf16);
+#undef RB_ONW
+#undef RB_ONR
+    }
+    // wider rows: a stack takes a thread per 16 bytes, so that all of a row's loads are in flight at once
     int threads = outnorm_threads(h);
-    if (vec && n_parts > 1) { threads = ((h / 4 + 31) / 32) * 32; if (threads > 1024) threads = 1024; if (threads < 128) threads = 128; }
+    if (vec && n_parts > 1) threads = 1024;
 #define RB_ON(TW, V) do { \
         if (smem > 48 * 1024) { \
             cudaError_t e = cudaFuncSetAttribute(residual_outnorm_kernel<TW, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
